@@ -50,6 +50,7 @@ struct FactorPlan {
   std::vector<int64_t> tile_level_ptr;  // host, nlevels+1
   DBuf<int2> trsm;             // (supernode, first row) chunks of the row solves
   std::vector<int64_t> trsm_level_ptr;
+  std::vector<int> level_width;  // host: widest supernode with rows below its block, per level
   int64_t n_trsm = 0;
   int64_t n_relind = 0;
   int64_t n_tiles = 0;

@@ -7,9 +7,9 @@
 //
 // Schedule: bottom-up levels of the supernodal elimination tree.  Per level:
 //   k_potrf      : one CTA per supernode: dense Cholesky of the (<=64 x 64)
-//                  diagonal block in shared memory;
-//   k_trsm       : the below-diagonal rows solved against it, 128 rows per
-//                  CTA (one row per thread, in registers);
+//                  diagonal block, 8 columns at a time;
+//   k_trsm       : the below-diagonal rows solved against it, 64 rows per
+//                  CTA, 16 columns at a time;
 //   k_update     : the Schur update L21 L21^T of every supernode of the level,
 //                  in 64x64 tiles on the FP64 tensor cores (DMMA
 //                  mma.sync.m8n8k4.f64), scattered into the ancestor panels
@@ -40,8 +40,6 @@ __global__ void k_load_A(int64_t n, const int* __restrict__ src, const int64_t* 
   L[dst[q]] = a * M[p] + (K ? b * K[p] : 0.0);
 }
 
-constexpr int kFacThreads = 128;
-
 // Dense Cholesky of the (<= 64 x 64) diagonal block of each supernode of a level.
 //
 // sgn != null: the indefinite mode, A = L S L^T with S = diag(+-1) (sgn, in
@@ -53,95 +51,226 @@ constexpr int kFacThreads = 128;
 // pivot is recorded in status[0] in both modes.
 constexpr double kPivotTol = 1e-13;
 
-__global__ void __launch_bounds__(kFacThreads) k_potrf(
+__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+constexpr int kPotrfThreads = 256;  // warps 0-1: the panel's rows; the others: the columns after it, finished columns out
+constexpr int kPanel = 8;           // columns eliminated between two trailing updates
+constexpr int kLdD = kSnCols + 2;   // row stride of the block in shared memory: column reads and DMMA fragments 2-way
+
+struct PotrfShared {
+  double D[kSnCols][kLdD];
+  double diag[kSnCols];  // L_kk
+  double dinv[kSnCols];  // 1 / L_kk
+  double sg[kSnCols];    // sign of the pivot (1 unless indefinite)
+  double d0[kSnCols];    // diagonal entries as the block's elimination starts
+};
+
+// Panel p, 8 columns, by warps 0 and 1: lane l of warp w owns row 32 w + l.
+//  1. The panel's entries get the rank-8 update of the panel before (earlier
+//     ones are in already), in registers.
+//  2. Every lane eliminates the panel's 8 x 8 diagonal block redundantly, so
+//     the chain per column is the square root, its reciprocal, a multiply and
+//     an FMA, with nothing to broadcast (a 64-bit shuffle issues in 11 cycles
+//     on sm_100a, a warp's FP64 FMA in 3).
+//  3. Each lane substitutes its own row.
+// Every entry gets the FMAs of column-by-column elimination in ascending
+// column order: the same rounding whatever the panel width.
+template <bool kIndef>
+__device__ __forceinline__ void potrf_panel(PotrfShared& S, int p, int c, int f, int* status, double* sgn) {
+  const int row = threadIdx.x, j0 = kPanel * p;  // threadIdx.x < 64
+  double a[kPanel];
+#pragma unroll
+  for (int k = 0; k < kPanel; ++k) a[k] = S.D[row][j0 + k];
+  if (p > 0) {
+    const int i0 = j0 - kPanel;
+    double l[kPanel];
+#pragma unroll
+    for (int k = 0; k < kPanel; ++k) l[k] = kIndef ? S.D[row][i0 + k] * S.sg[i0 + k] : S.D[row][i0 + k];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j)
+#pragma unroll
+      for (int k = 0; k < kPanel; ++k) a[j] -= l[k] * S.D[j0 + j][i0 + k];
+#pragma unroll
+    for (int k = 0; k < kPanel; ++k)
+      if (row >= j0 && row < j0 + kPanel) S.D[row][j0 + k] = a[k];
+  }
+  asm volatile("bar.sync 1, 64;\n" ::: "memory");
+  double t[kPanel][kPanel], inv[kPanel], sg[kPanel], mydiag = 0.0, myinv = 0.0, mysg = 1.0;
+#pragma unroll
+  for (int i = 0; i < kPanel; ++i)
+#pragma unroll
+    for (int k = 0; k <= i; ++k) t[i][k] = S.D[j0 + i][j0 + k];
+  int bad = INT_MAX, npert = 0;
+#pragma unroll
+  for (int k = 0; k < kPanel; ++k) {
+    double d = t[k][k];
+    sg[k] = 1.0;
+    if (!(d > 0.0) && j0 + k < c) bad = min(bad, j0 + k);  // non-positive or NaN pivot
+    if (kIndef) {
+      sg[k] = d < 0.0 ? -1.0 : 1.0;
+      d = fabs(d);
+      const double d0 = S.d0[j0 + k];
+      const double tau = kPivotTol * (d0 > 0.0 ? d0 : 1.0);
+      if (!(d >= tau) || !(d <= 1e300)) {  // cancelled, NaN or infinite pivot: perturb
+        d = tau;
+        npert += j0 + k < c ? 1 : 0;
+      }
+    } else {
+      d = d > 0.0 ? d : 1.0;  // continue with 1; the factor is reported invalid
+    }
+    const double lkk = sqrt(d);
+    inv[k] = 1.0 / lkk;
+    if (row == j0 + k) {
+      mydiag = lkk;
+      myinv = inv[k];
+      mysg = sg[k];
+    }
+    if (kIndef) inv[k] *= sg[k];
+#pragma unroll
+    for (int i = k + 1; i < kPanel; ++i) t[i][k] *= inv[k];
+#pragma unroll
+    for (int j = k + 1; j < kPanel; ++j)
+#pragma unroll
+      for (int i = j; i < kPanel; ++i) t[i][j] -= (kIndef ? t[i][k] * sg[k] : t[i][k]) * t[j][k];
+  }
+#pragma unroll
+  for (int k = 0; k < kPanel; ++k) {
+    a[k] *= inv[k];
+#pragma unroll
+    for (int j = k + 1; j < kPanel; ++j) a[j] -= (kIndef ? a[k] * sg[k] : a[k]) * t[j][k];
+  }
+  asm volatile("bar.sync 1, 64;\n" ::: "memory");  // the diagonal block has been read
+#pragma unroll
+  for (int k = 0; k < kPanel; ++k)
+    if (row > j0 + k) S.D[row][j0 + k] = a[k];
+  if (row >= j0 && row < j0 + kPanel) {
+    S.diag[row] = mydiag;
+    S.dinv[row] = myinv;
+    S.sg[row] = mysg;
+    if (kIndef && row < c) sgn[f + row] = mysg;
+  }
+  if (row == 0) {
+    if (bad != INT_MAX) atomicMin(status, f + bad + 1);
+    if (kIndef && npert) atomicAdd(status + 2, npert);
+  }
+}
+
+// Tile (I, J) of 8 x 8 minus the products with panel p.  The tile is the
+// accumulator: a DMMA adds its four products one FMA after the other in
+// ascending k, as column-by-column elimination does.
+__device__ __forceinline__ void potrf_tile(PotrfShared& S, int I, int J, int p) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int ri = 8 * I + g, rj = 8 * J;
+  double x0 = S.D[ri][rj + 2 * q], x1 = S.D[ri][rj + 2 * q + 1];
+#pragma unroll
+  for (int k0 = 0; k0 < kPanel; k0 += 4) {
+    const int k = kPanel * p + k0 + q;
+    dmma_8x8x4(x0, x1, -S.D[ri][k] * S.sg[k], S.D[rj + g][k]);
+  }
+  S.D[ri][rj + 2 * q] = x0;
+  S.D[ri][rj + 2 * q + 1] = x1;
+}
+
+// One CTA per block, bound by the 64-step pivot chain.  While warps 0 and 1
+// eliminate panel p, the others apply panel p - 1 to the columns after p
+// (DMMA) and write the finished columns of panel p - 1: the panel's block, and
+// the sweeps' copy (row i scaled by 1/L_ii, 1/L_ii on the diagonal, zeros
+// above; c x c, column-major).  A 64 x 64 block in its stream takes 14.4 us;
+// column by column with two barriers, a square root and a division per
+// column it took 73.  Two CTAs per SM: the bottom levels hold hundreds of
+// narrow blocks.
+template <bool kIndef>
+__global__ void __launch_bounds__(kPotrfThreads, 2) k_potrf(
     const int* __restrict__ level_sn, const int* __restrict__ sn_first,
     const int64_t* __restrict__ rows_ptr, const int64_t* __restrict__ Lptr, double* __restrict__ L,
     int* __restrict__ status, double* __restrict__ sgn, const int64_t* __restrict__ Dptr) {
-  constexpr int CB = kSnCols;
-  __shared__ double D[CB][CB + 1];
-  __shared__ double diag[CB];  // L_kk, written into D after the loop
-  __shared__ double d0[CB];
+  __shared__ PotrfShared S;
   const int s = level_sn[blockIdx.x];
   const int f = sn_first[s];
   const int c = sn_first[s + 1] - f;
   const int64_t r = rows_ptr[s + 1] - rows_ptr[s];
   const int64_t ld = c + r;
   double* P = L + Lptr[s];
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx % c;
-    D[i][j] = (i >= j) ? P[(int64_t)j * ld + i] : 0.0;
-  }
-  __syncthreads();
-  if (tid < c) d0[tid] = fabs(D[tid][tid]);
-  __syncthreads();
-  // Right-looking, two barriers per column: every thread derives the pivot
-  // from the same shared value (the diagonal itself is written at the end),
-  // the column is scaled, then the trailing triangle is updated on a 8 x 16
-  // thread grid.
-  const int tx = tid & 15, ty = tid >> 4;
-  for (int k = 0; k < c; ++k) {
-    const double a = D[k][k];
-    double d = a, s = 1.0;
-    bool perturbed = false;
-    if (sgn) {
-      s = d < 0.0 ? -1.0 : 1.0;
-      d = fabs(d);
-      const double tau = kPivotTol * (d0[k] > 0.0 ? d0[k] : 1.0);
-      if (!(d >= tau) || !(d <= 1e300)) {  // cancelled, NaN or infinite pivot: perturb
-        d = tau;
-        perturbed = true;
-      }
-    } else if (!(d > 0.0)) {
-      d = 1.0;  // continue with 1; the factor is reported invalid
-    }
-    const double lkk = sqrt(d);
-    if (tid == 0) {
-      if (!(a > 0.0)) atomicMin(status, f + k + 1);  // non-positive or NaN pivot: record
-      if (perturbed) atomicAdd(status + 2, 1);
-      if (sgn) sgn[f + k] = s;
-      diag[k] = lkk;
-    }
-    const double inv = 1.0 / (lkk * s);
-    for (int i = k + 1 + tid; i < c; i += blockDim.x) D[i][k] *= inv;
-    __syncthreads();
-    for (int ii = k + 1 + ty; ii < c; ii += 8) {
-      const double lik = D[ii][k] * s;
-      for (int jj = k + 1 + tx; jj <= ii; jj += 16) D[ii][jj] -= lik * D[jj][k];
-    }
-    __syncthreads();
-  }
-  if (tid < c) {
-    D[tid][tid] = diag[tid];
-    d0[tid] = 1.0 / diag[tid];
-  }
-  __syncthreads();
-  // the panel's block, and the sweeps' copy: row i scaled by 1/L_ii, 1/L_ii on
-  // the diagonal, zeros above (c x c, column-major)
   double* Q = L + Dptr[s];
-  for (int idx = tid; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx % c;
-    if (i >= j) P[(int64_t)j * ld + i] = D[i][j];
-    Q[idx] = i > j ? D[i][j] * d0[i] : (i == j ? d0[i] : 0.0);
+  const int tid = threadIdx.x, i = tid & (kSnCols - 1);
+  const int np = (c + kPanel - 1) / kPanel;
+  // lower triangle; zeros above it and past c
+#pragma unroll 16
+  for (int j = tid / kSnCols; j < np * kPanel; j += kPotrfThreads / kSnCols)
+    S.D[i][j] = (i < c && j <= i) ? P[(int64_t)j * ld + i] : 0.0;
+  if (tid < kSnCols) S.sg[tid] = 1.0;
+  __syncthreads();
+  if (kIndef) {
+    if (tid < c) S.d0[tid] = fabs(S.D[tid][tid]);
+    __syncthreads();
+  }
+  // columns of panel p out, by `nt` threads from `t0` on
+  auto out = [&](int p, int t0, int nt) {
+    if (i >= c) return;
+    for (int j = kPanel * p + (tid - t0) / kSnCols; j < min(c, kPanel * (p + 1)); j += nt / kSnCols)
+      if (i >= j) P[(int64_t)j * ld + i] = i > j ? S.D[i][j] : S.diag[i];
+  };
+  for (int p = 0; p <= np; ++p) {
+    if (tid < 64) {
+      if (p < np) potrf_panel<kIndef>(S, p, c, f, status, sgn);
+    } else if (p > 0) {
+      int t = (tid >> 5) - 2;
+      for (int J = p + 1; J < np; ++J)
+        for (int I = J; I < np; ++I, ++t)
+          if (t % 6 == 0) potrf_tile(S, I, J, p - 1);
+      out(p - 1, 64, kPotrfThreads - 64);
+    }
+    __syncthreads();
+  }
+  if (i < c) {
+    const double di = S.dinv[i];
+    for (int j = tid / kSnCols; j < c; j += kPotrfThreads / kSnCols)
+      Q[(int64_t)j * c + i] = i > j ? S.D[i][j] * di : (i == j ? di : 0.0);
   }
 }
 
+// a / b correctly rounded, from y = 1 / b correctly rounded: two residual
+// corrections of a y, the last of which rounds correctly (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990, theorem on quotients) while neither
+// over- nor underflows.  45 cycles on the chain of a row, a division 110.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+
 // Below-diagonal rows of the level's supernodes, kTrsmRows rows per CTA:
-// x L11^T = a, forward substitution per row in registers.
+// x L11^T = a, L21 = x S11 in the indefinite mode (sgn != null).  Panels of 16
+// columns: the products with the columns before a panel are DMMA tiles that
+// start from the panel's entries (each entry gets its FMAs in ascending
+// column order, as in a row-by-row substitution), then one thread per row
+// substitutes inside the panel in registers.  A level of one 64-column block
+// takes 12.5 us where one row per thread and a division per column took 36.
 struct TrsmChunk {
   int s;
   int r0;
 };
-constexpr int kTrsmRows = kFacThreads;
+constexpr int kTrsmRows = 64;
+constexpr int kTrsmThreads = 128;
+constexpr int kTrsmPanel = 16;
+constexpr int kLdX = kTrsmRows + 4;         // DMMA fragments (4 columns x 8 rows) without bank conflicts
 
-// Indefinite mode (sgn != null): L21 = A21 L11^{-T} S11.
-__global__ void __launch_bounds__(kFacThreads) k_trsm(const TrsmChunk* __restrict__ chunks,
-                                                      const int* __restrict__ sn_first,
-                                                      const int64_t* __restrict__ rows_ptr,
-                                                      const int64_t* __restrict__ Lptr, double* __restrict__ L,
-                                                      const double* __restrict__ sgn) {
-  constexpr int CB = kSnCols;
-  __shared__ double D[CB][CB + 1];
+inline size_t trsm_smem(int width) {        // X [w][kLdX], the block [w][kLdD], 1 / L_kk [w]; w: whole panels
+  const int w = (width + kTrsmPanel - 1) / kTrsmPanel * kTrsmPanel;
+  return (size_t)w * (kLdX + kLdD + 1) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restrict__ chunks,
+                                                       const int* __restrict__ sn_first,
+                                                       const int64_t* __restrict__ rows_ptr,
+                                                       const int64_t* __restrict__ Lptr, double* __restrict__ L,
+                                                       const double* __restrict__ sgn) {
+  extern __shared__ __align__(16) double trsm_sm[];
   const TrsmChunk ch = chunks[blockIdx.x];
   const int s = ch.s;
   const int f = sn_first[s];
@@ -149,40 +278,73 @@ __global__ void __launch_bounds__(kFacThreads) k_trsm(const TrsmChunk* __restric
   const int64_t r = rows_ptr[s + 1] - rows_ptr[s];
   const int64_t ld = c + r;
   double* P = L + Lptr[s];
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx % c;
-    if (i >= j) D[i][j] = P[(int64_t)j * ld + i];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int np = (c + kTrsmPanel - 1) / kTrsmPanel, w = np * kTrsmPanel;
+  double* X = trsm_sm;              // [column][row]
+  double* D = X + w * kLdX;         // [row of L11][column]; past c: zeros, ones on the diagonal
+  double* rinv = D + w * kLdD;
+  const int t = tid & (kTrsmRows - 1);
+  const int64_t i = ch.r0 + t;
+  const bool on = i < r;
+  double* row = P + c + i;
+#pragma unroll 8
+  for (int j = tid / kTrsmRows; j < w; j += kTrsmThreads / kTrsmRows) {
+    const double x = (on && j < c) ? row[(int64_t)j * ld] : 0.0;
+    const double d = (t >= j && t < c) ? P[(int64_t)j * ld + t] : (t == j ? 1.0 : 0.0);
+    X[j * kLdX + t] = x;
+    if (t < w) D[t * kLdD + j] = d;
   }
   __syncthreads();
-  const int64_t i = ch.r0 + tid;
-  if (i >= r) return;
-  double x[CB];
+  if (tid < w) rinv[tid] = 1.0 / D[tid * kLdD + tid];
+  __syncthreads();
+  for (int p = 0; p < np; ++p) {
+    const int j0 = kTrsmPanel * p;
+    if (p > 0) {  // rows 16 warp .. + 15 of the panel minus the products with the columns before it
+      double acc[2][2][2];
 #pragma unroll
-  for (int j = 0; j < CB; ++j) x[j] = (j < c) ? P[(int64_t)j * ld + c + i] : 0.0;
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-  for (int j = 0; j < CB; ++j) {
-    if (j < c) {
-      double v = x[j];
+        for (int b = 0; b < 2; ++b)
 #pragma unroll
-      for (int k = 0; k < j; ++k) v -= x[k] * D[j][k];
-      x[j] = v / D[j][j];
+          for (int e = 0; e < 2; ++e) acc[a][b][e] = X[(j0 + 8 * b + 2 * q + e) * kLdX + 16 * warp + 8 * a + g];
+#pragma unroll 4
+      for (int k0 = 0; k0 < j0; k0 += 4) {
+        double fa[2], fb[2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a) fa[a] = -X[(k0 + q) * kLdX + 16 * warp + 8 * a + g];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) fb[b] = D[(j0 + 8 * b + g) * kLdD + k0 + q];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+      }
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) X[(j0 + 8 * b + 2 * q + e) * kLdX + 16 * warp + 8 * a + g] = acc[a][b][e];
+      __syncthreads();
     }
-  }
-  if (sgn) {
+    if (tid < kTrsmRows) {
+      double x[kTrsmPanel];
 #pragma unroll
-    for (int j = 0; j < CB; ++j)
-      if (j < c) x[j] *= sgn[f + j];
-  }
+      for (int j = 0; j < kTrsmPanel; ++j) x[j] = X[(j0 + j) * kLdX + t];
 #pragma unroll
-  for (int j = 0; j < CB; ++j)
-    if (j < c) P[(int64_t)j * ld + c + i] = x[j];
-}
-
-__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
+      for (int j = 0; j < kTrsmPanel; ++j) {
+        x[j] = quotient(x[j], D[(j0 + j) * kLdD + j0 + j], rinv[j0 + j]);
+#pragma unroll
+        for (int k = j + 1; k < kTrsmPanel; ++k) x[k] -= x[j] * D[(j0 + k) * kLdD + j0 + j];
+      }
+#pragma unroll
+      for (int j = 0; j < kTrsmPanel; ++j) {
+        X[(j0 + j) * kLdX + t] = x[j];
+        if (on && j0 + j < c) row[(int64_t)(j0 + j) * ld] = sgn ? x[j] * sgn[f + j0 + j] : x[j];
+      }
+    }
+    __syncthreads();
+  }
 }
 
 constexpr int kLdsU = kUpdTile + 8;  // 72 doubles: two 128-byte wavefronts per fragment load
@@ -484,11 +646,13 @@ void build_factor_plan(temf_ctx& c) {
   {
     std::vector<TrsmChunk> ch;
     std::vector<int64_t> lp(S.nlevels + 1, 0);
+    F.level_width.assign(S.nlevels, 0);
     for (int l = 0; l < S.nlevels; ++l) {
       for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
         const int s = S.level_sn[q];
         const int r = (int)nrows(s);
         for (int r0 = 0; r0 < r; r0 += kTrsmRows) ch.push_back({s, r0});
+        F.level_width[l] = std::max(F.level_width[l], width(s));
       }
       lp[l + 1] = (int64_t)ch.size();
     }
@@ -604,17 +768,19 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   }
   const size_t upd_smem = 2 * 2 * kUpdChunk * kLdsU * sizeof(double);
   TEMF_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)upd_smem));
+  TEMF_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(kSnCols)));
   for (int l = 0; l < S.nlevels; ++l) {
     const int cnt = S.level_ptr[l + 1] - S.level_ptr[l];
     if (cnt > 0) {
-      k_potrf<<<cnt, kFacThreads, 0, st>>>(F.level_sn.p + S.level_ptr[l], F.sn_first.p, F.sn_rows_ptr.p,
-                                           F.sn_Lptr.p, fs.L.p, c.d_status.p, sgn, F.sn_Dptr.p);
+      const auto potrf = indefinite ? k_potrf<true> : k_potrf<false>;
+      potrf<<<cnt, kPotrfThreads, 0, st>>>(F.level_sn.p + S.level_ptr[l], F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p,
+                                           fs.L.p, c.d_status.p, sgn, F.sn_Dptr.p);
       TEMF_CHECK_LAUNCH();
     }
     const int64_t c0 = F.trsm_level_ptr[l], c1 = F.trsm_level_ptr[l + 1];
     if (c1 > c0) {
-      k_trsm<<<(unsigned)(c1 - c0), kFacThreads, 0, st>>>(reinterpret_cast<const TrsmChunk*>(F.trsm.p) + c0,
-                                                          F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p, fs.L.p, sgn);
+      k_trsm<<<(unsigned)(c1 - c0), kTrsmThreads, trsm_smem(F.level_width[l]), st>>>(
+          reinterpret_cast<const TrsmChunk*>(F.trsm.p) + c0, F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p, fs.L.p, sgn);
       TEMF_CHECK_LAUNCH();
     }
     const int64_t t0 = F.tile_level_ptr[l], t1 = F.tile_level_ptr[l + 1];
