@@ -51,6 +51,7 @@ struct FactorPlan {
   DBuf<int2> trsm;             // (supernode, first row) chunks of the row solves
   std::vector<int64_t> trsm_level_ptr;
   std::vector<int> level_width;  // host: widest supernode with rows below its block, per level
+  std::vector<int> upd_shape;    // host: shape of each level's update kernel (factor.cu)
   int64_t n_trsm = 0;
   int64_t n_relind = 0;
   int64_t n_tiles = 0;

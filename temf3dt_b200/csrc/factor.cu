@@ -347,8 +347,6 @@ __global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restri
   }
 }
 
-constexpr int kLdsU = kUpdTile + 8;  // 72 doubles: two 128-byte wavefronts per fragment load
-
 // Bulk global -> shared copies on the TMA engine (cp.async.bulk, this GPU's
 // own memory, each CTA its own copy), completed on an mbarrier: one instruction per
 // panel column segment instead of one 8-byte copy per element.  Addresses
@@ -397,34 +395,53 @@ __device__ __forceinline__ void mbar_wait(uint64_t* b, unsigned parity, int* err
 
 // Schur update tiles.  A tile (s, i0, j0, members m, column limit jl) holds
 // C = sum over the m supernodes q = s-m+1 .. s of L21_q[rows beyond] *
-// L21_q[rows beyond]^T for the 64 x 64 block (i0.., j0..) of s's row list:
+// L21_q[rows beyond]^T for the kT x kT block (i0.., j0..) of s's row list:
 // m > 1 for the column blocks of one wider supernode (a run), whose updates
 // beyond the run are summed in one pass (K = the run's columns, each member's
 // rows beyond the run are the rows of s, at offset r_q - r_s of its list);
 // m = 1 otherwise.  jl > 0 restricts the tile to columns j < jl (inside a run,
 // a member updates the later members' columns only).  C is scattered into the
-// ancestors' panels through the relative indices of s.  The K loop runs over
-// 16-column chunks of the members, double-buffered: the next chunk's bulk
-// copies (one per column segment of A and of B: 32 per chunk, issued by warp
-// 0) are in flight while the DMMA tiles consume the current one (37 KB of
-// shared memory: five CTAs per SM, by registers, where 32-column chunks
-// allowed three).
+// ancestors' panels through the relative indices of s, one red.global.add per
+// entry (no read comes back to wait for; a level of several supernodes needs
+// atomics anyway).  The K loop runs over 16-column chunks of the members
+// through kStages buffers: bulk copies (one per column segment of A and of B:
+// 32 per chunk, issued by warp 0) are in flight while the DMMA tiles consume
+// the current chunk; the targets of the tile's columns are looked up
+// meanwhile.
+//
+// Tile size and buffers go by the tiles of the level (update_shape): a level
+// that gives every SM several 64 x 64 tiles is bound by the FP64 tensor pipe
+// and runs two buffers, five CTAs per SM; a smaller level is bound by the
+// latency of one tile, and four buffers hide the copies' (a 64 x 64 tile of
+// 512 columns on its own: 83 us with two buffers and a read-modify-write
+// scatter, 49 as 32 x 32 tiles); one that leaves SMs without a tile runs 32 x 32 tiles, four times
+// as many and a quarter as long.  An entry's sum runs over the same columns
+// in the same order in every shape.
 constexpr int kUpdChunk = 16;
 constexpr int kUpdMaxMembers = 8;
 
-__global__ void __launch_bounds__(128, 5) k_update(
+template <int kT, int kStages>
+constexpr size_t update_smem() {
+  return (size_t)kStages * 2 * kUpdChunk * (kT + 4) * sizeof(double);
+}
+
+template <int kT, int kStages>
+__global__ void __launch_bounds__(128, kStages == 2 ? 5 : 3) k_update(
     const UpdTile* __restrict__ tiles, const int* __restrict__ sn_first,
     const int64_t* __restrict__ rows_ptr, const int* __restrict__ sn_rows,
     const int64_t* __restrict__ Lptr, const int* __restrict__ row_grp,
     const int* __restrict__ grp_target, const int* __restrict__ grp_shift,
     const int64_t* __restrict__ grp_relind, const int* __restrict__ relind, double* __restrict__ L,
-    int use_atomics, const double* __restrict__ sgn, int* __restrict__ err) {
+    const double* __restrict__ sgn, int* __restrict__ err) {
+  constexpr int kLd = kT + 4;   // fragment loads (4 columns x 8 rows) without bank conflicts; room for the shift
+  constexpr int kF = kT / 16;   // 8-wide fragments per warp and side: warps 2 x 2 of kT/2 x kT/2
   extern __shared__ __align__(128) double sm[];
-  __shared__ __align__(8) uint64_t mbar[2];
-  __shared__ unsigned char shift[2][2][kUpdChunk];  // per buffer, operand, row: offset of the segment's first row
-  // [buffer][A | B][kUpdChunk][kLdsU]
-  auto As = [&](int buf) { return sm + (size_t)buf * 2 * kUpdChunk * kLdsU; };
-  auto Bs = [&](int buf) { return sm + (size_t)buf * 2 * kUpdChunk * kLdsU + kUpdChunk * kLdsU; };
+  __shared__ __align__(8) uint64_t mbar[kStages];
+  __shared__ unsigned char shift[kStages][2][kUpdChunk];  // per buffer, operand, row: offset of the segment's first row
+  __shared__ int64_t tcol[kT], trel[kT];                  // per column: its target column, its relative indices
+  // [buffer][A | B][kUpdChunk][kLd]
+  auto As = [&](int buf) { return sm + (size_t)buf * 2 * kUpdChunk * kLd; };
+  auto Bs = [&](int buf) { return sm + (size_t)buf * 2 * kUpdChunk * kLd + kUpdChunk * kLd; };
   const UpdTile tile = tiles[blockIdx.x];
   const int s = tile.s;
   const int m = tile.mj & 15;
@@ -448,7 +465,7 @@ __global__ void __launch_bounds__(128, 5) k_update(
       k0 = 0;
     }
   };
-  auto issue = [&](int buf) {
+  auto issue = [&](int buf) {  // warp 0
     const int q = cp_q, k0 = cp_k0;
     advance(cp_q, cp_k0);
     const int fq = sn_first[q];
@@ -456,102 +473,119 @@ __global__ void __launch_bounds__(128, 5) k_update(
     const int rq = (int)(rows_ptr[q + 1] - rows_ptr[q]);
     const int64_t ldq = cq + rq;
     const double* P = L + Lptr[q] + cq + (rq - r);  // row 0 of the rows beyond the run
-    if (tid < 2 * kUpdChunk) {  // warp 0: one segment each (operand A rows i0.., B rows j0..)
-      const int op = tid / kUpdChunk, k = tid % kUpdChunk, kk = k0 + k;
-      const int g0 = op == 0 ? tile.i0 : tile.j0;
-      double* row = (op == 0 ? As(buf) : Bs(buf)) + k * kLdsU;
-      if (kk < cq && g0 < r) {
-        const double* src = P + (int64_t)kk * ldq + g0;
-        const int n = min(kUpdTile, r - g0);  // rows past r only feed outputs that are not scattered
-        const int o = (__cvta_generic_to_global(src) & 15) ? 1 : 0;
-        const unsigned bytes = (unsigned)(((n + o) * 8 + 15) & ~15);
-        shift[buf][op][k] = (unsigned char)o;
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        mbar_expect_tx(&mbar[buf], bytes);
-        bulk_g2s(row, src - o, bytes, &mbar[buf]);
-      } else {  // past the member's columns: a zero row
-        shift[buf][op][k] = 0;
-        for (int ii = 0; ii < kUpdTile; ++ii) row[ii] = 0.0;
-      }
-      __syncwarp();
-      if (tid == 0) mbar_arrive(&mbar[buf]);
+    // one segment per lane (operand A rows i0.., B rows j0..)
+    const int op = tid / kUpdChunk, k = tid % kUpdChunk, kk = k0 + k;
+    const int g0 = op == 0 ? tile.i0 : tile.j0;
+    double* row = (op == 0 ? As(buf) : Bs(buf)) + k * kLd;
+    if (kk < cq && g0 < r) {
+      const double* src = P + (int64_t)kk * ldq + g0;
+      const int n = min(kT, r - g0);  // rows past r only feed outputs that are not scattered
+      const int o = (__cvta_generic_to_global(src) & 15) ? 1 : 0;
+      const unsigned bytes = (unsigned)(((n + o) * 8 + 15) & ~15);
+      shift[buf][op][k] = (unsigned char)o;
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      mbar_expect_tx(&mbar[buf], bytes);
+      bulk_g2s(row, src - o, bytes, &mbar[buf]);
+    } else {  // past the member's columns: a zero row
+      shift[buf][op][k] = 0;
+      for (int ii = 0; ii < kT; ++ii) row[ii] = 0.0;
     }
+    __syncwarp();
+    if (tid == 0) mbar_arrive(&mbar[buf]);
   };
   const int warp = tid >> 5, lane = tid & 31;
-  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
+  const int wr = (warp >> 1) * (kT / 2), wc = (warp & 1) * (kT / 2);
   const int g = lane >> 2, qd = lane & 3;
-  double acc[4][4][2];
+  double acc[kF][kF][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < kF; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < kF; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
   if (tid == 0) {
-    mbar_init(&mbar[0], 1);
-    mbar_init(&mbar[1], 1);
+#pragma unroll
+    for (int u = 0; u < kStages; ++u) mbar_init(&mbar[u], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int u = 0; u < kStages - 1; ++u)
+      if (u < nch) issue(u);
+  }
+  // scatter targets of the tile's columns (read after the K loop's barriers)
+  const int jend = jl > 0 ? min(jl, r) : r;
+  if (tid >= 128 - kT) {
+    const int jj = tid - (128 - kT), j = tile.j0 + jj;
+    if (j < jend) {
+      const int grp = row_grp[rp + j];
+      const int t = grp_target[grp];
+      const int ft = sn_first[t];
+      const int64_t ldt = sn_first[t + 1] - ft + (rows_ptr[t + 1] - rows_ptr[t]);
+      tcol[jj] = Lptr[t] + (int64_t)(sn_rows[rp + j] - ft) * ldt - grp_shift[grp];
+      trel[jj] = grp_relind[grp];
+    }
+  }
   unsigned phases = 0u;  // bit b: parity of buffer b's next phase
-  issue(0);
+  int buf = 0;
   for (int ch = 0; ch < nch; ++ch) {
-    const int buf = ch & 1;
-    if (ch + 1 < nch) issue(buf ^ 1);
     mbar_wait(&mbar[buf], (phases >> buf) & 1u, err);
     phases ^= 1u << buf;
-    __syncthreads();
+    __syncthreads();  // the chunk before has been consumed: its buffer is free
+    if (warp == 0 && ch + kStages - 1 < nch) issue(buf == 0 ? kStages - 1 : buf - 1);
     double* A = As(buf);
     const double* B = Bs(buf);
     if (sgn) {  // indefinite mode: A22 -= L21 S11 L21^T
       const int fq = sn_first[mm_q];
       const int cq = sn_first[mm_q + 1] - fq;
-      for (int idx = tid; idx < kUpdChunk * kUpdTile; idx += blockDim.x) {
-        const int k = idx / kUpdTile, ii = idx % kUpdTile;
-        if (mm_k0 + k < cq) A[k * kLdsU + shift[buf][0][k] + ii] *= sgn[fq + mm_k0 + k];
+      for (int idx = tid; idx < kUpdChunk * kT; idx += blockDim.x) {
+        const int k = idx / kT, ii = idx % kT;
+        if (mm_k0 + k < cq) A[k * kLd + shift[buf][0][k] + ii] *= sgn[fq + mm_k0 + k];
       }
       __syncthreads();
+      advance(mm_q, mm_k0);
     }
-    advance(mm_q, mm_k0);
 #pragma unroll 2
     for (int k0 = 0; k0 < kUpdChunk; k0 += 4) {
-      double fa[4], fb[4];
+      double fa[kF], fb[kF];
       const int sa = shift[buf][0][k0 + qd], sb = shift[buf][1][k0 + qd];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) fa[a] = A[(k0 + qd) * kLdsU + sa + wr + a * 8 + g];
+      for (int a = 0; a < kF; ++a) fa[a] = A[(k0 + qd) * kLd + sa + wr + a * 8 + g];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) fb[b] = B[(k0 + qd) * kLdsU + sb + wc + b * 8 + g];
+      for (int b = 0; b < kF; ++b) fb[b] = B[(k0 + qd) * kLd + sb + wc + b * 8 + g];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < kF; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+        for (int b = 0; b < kF; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
     }
-    __syncthreads();  // the buffer is refilled by the next issue
+    buf = buf == kStages - 1 ? 0 : buf + 1;
   }
   // scatter-subtract into the ancestors
-  const int jend = jl > 0 ? min(jl, r) : r;
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
+  for (int b = 0; b < kF; ++b) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int j = tile.j0 + wc + b * 8 + 2 * qd + e;
+      const int jj = wc + b * 8 + 2 * qd + e, j = tile.j0 + jj;
       if (j >= jend) continue;
-      const int grp = row_grp[rp + j];
-      const int t = grp_target[grp];
-      const int ft = sn_first[t];
-      const int ct = sn_first[t + 1] - ft;
-      const int64_t ldt = ct + (rows_ptr[t + 1] - rows_ptr[t]);
-      double* dstcol = L + Lptr[t] + (int64_t)(sn_rows[rp + j] - ft) * ldt - grp_shift[grp];
-      const int* rel = relind + grp_relind[grp];
+      double* dst = L + tcol[jj];
+      const int* rel = relind + trel[jj];
+      int at[kF];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
+      for (int a = 0; a < kF; ++a) {
         const int i = tile.i0 + wr + a * 8 + g;
-        if (i < r && i >= j) {
-          // one supernode per level: every target entry has a single writer
-          if (use_atomics) atomicAdd(dstcol + rel[i], -acc[a][b][e]);
-          else dstcol[rel[i]] -= acc[a][b][e];
-        }
+        at[a] = i < r && i >= j ? rel[i] : -1;
       }
+#pragma unroll
+      for (int a = 0; a < kF; ++a)
+        if (at[a] >= 0) atomicAdd(dst + at[a], -acc[a][b][e]);
     }
   }
+}
+
+// Shape of a level's update kernel by its number of 64 x 64 tiles.
+enum UpdShape { kUpdWide = 0, kUpdDeep = 1, kUpdSmall = 2 };
+constexpr int kSms = 148;
+inline UpdShape update_shape(int64_t tiles64) {
+  return tiles64 >= 8 * kSms ? kUpdWide : (tiles64 >= kSms ? kUpdDeep : kUpdSmall);
 }
 
 // ---------------------------------------------------------------------------
@@ -666,7 +700,8 @@ void build_factor_plan(temf_ctx& c) {
     F.n_runs = 0;
     std::vector<UpdTile> tiles;
     F.tile_level_ptr.assign(S.nlevels + 1, 0);
-    for (int l = 0; l < S.nlevels; ++l) {
+    // tiles of level l with edge T appended
+    auto level_tiles = [&](int l, int T, std::vector<UpdTile>& out, bool count_runs) {
       for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
         const int s = S.level_sn[q];
         const int r = (int)nrows(s);
@@ -674,16 +709,26 @@ void build_factor_plan(temf_ctx& c) {
         if (e != s) {
           // a run member before its last: only the later members' columns
           const int g = S.sn_first[e + 1] - S.sn_first[s + 1];
-          for (int tj = 0; tj * kUpdTile < g; ++tj)
-            for (int ti = tj; ti * kUpdTile < r; ++ti) tiles.push_back({s, ti * kUpdTile, tj * kUpdTile, 1 | (g << 4)});
+          for (int tj = 0; tj * T < g; ++tj)
+            for (int ti = tj; ti * T < r; ++ti) out.push_back({s, ti * T, tj * T, 1 | (g << 4)});
           continue;
         }
         int m = 1;  // members of the run ending at s
         while (s - m >= 0 && run_end[s - m] == s) ++m;
-        if (m > 1) ++F.n_runs;
-        const int nt = ceil_div(r, kUpdTile);
+        if (m > 1 && count_runs) ++F.n_runs;
+        const int nt = ceil_div(r, T);
         for (int ti = 0; ti < nt; ++ti)
-          for (int tj = 0; tj <= ti; ++tj) tiles.push_back({s, ti * kUpdTile, tj * kUpdTile, m});
+          for (int tj = 0; tj <= ti; ++tj) out.push_back({s, ti * T, tj * T, m});
+      }
+    };
+    F.upd_shape.assign(S.nlevels, kUpdWide);
+    for (int l = 0; l < S.nlevels; ++l) {
+      const size_t t0 = tiles.size();
+      level_tiles(l, kUpdTile, tiles, true);
+      F.upd_shape[l] = update_shape((int64_t)(tiles.size() - t0));
+      if (F.upd_shape[l] == kUpdSmall) {
+        tiles.resize(t0);
+        level_tiles(l, kUpdTile / 2, tiles, false);
       }
       F.tile_level_ptr[l + 1] = (int64_t)tiles.size();
     }
@@ -766,8 +811,11 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
     k_load_A<<<ceil_div(F.n_a2l, 256), 256, 0, st>>>(F.n_a2l, F.a2l_src.p, F.a2l_dst.p, X, a, Y, b, fs.L.p);
     TEMF_CHECK_LAUNCH();
   }
-  const size_t upd_smem = 2 * 2 * kUpdChunk * kLdsU * sizeof(double);
-  TEMF_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)upd_smem));
+  const auto upd_wide = k_update<kUpdTile, 2>;
+  const auto upd_deep = k_update<kUpdTile, 4>;
+  const auto upd_small = k_update<kUpdTile / 2, 4>;
+  TEMF_CUDA(cudaFuncSetAttribute(upd_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<kUpdTile, 2>()));
+  TEMF_CUDA(cudaFuncSetAttribute(upd_deep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<kUpdTile, 4>()));
   TEMF_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(kSnCols)));
   for (int l = 0; l < S.nlevels; ++l) {
     const int cnt = S.level_ptr[l + 1] - S.level_ptr[l];
@@ -786,10 +834,13 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
     const int64_t t0 = F.tile_level_ptr[l], t1 = F.tile_level_ptr[l + 1];
     if (t1 > t0) {
       if (t1 - t0 > INT_MAX) throw StateError("too many update tiles in one level");
-      k_update<<<(unsigned)(t1 - t0), 128, upd_smem, st>>>(F.tiles.p + t0, F.sn_first.p, F.sn_rows_ptr.p,
-                                                          F.sn_rows.p, F.sn_Lptr.p, F.row_grp.p, F.grp_target.p,
-                                                          F.grp_shift.p, F.grp_relind.p, F.relind.p, fs.L.p,
-                                                          cnt > 1 ? 1 : 0, sgn, c.d_status.p + 3);
+      const int sh = F.upd_shape[l];
+      const auto upd = sh == kUpdWide ? upd_wide : (sh == kUpdDeep ? upd_deep : upd_small);
+      const size_t smem = sh == kUpdWide ? update_smem<kUpdTile, 2>()
+                                         : (sh == kUpdDeep ? update_smem<kUpdTile, 4>() : update_smem<kUpdTile / 2, 4>());
+      upd<<<(unsigned)(t1 - t0), 128, smem, st>>>(F.tiles.p + t0, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p,
+                                                  F.sn_Lptr.p, F.row_grp.p, F.grp_target.p, F.grp_shift.p,
+                                                  F.grp_relind.p, F.relind.p, fs.L.p, sgn, c.d_status.p + 3);
       TEMF_CHECK_LAUNCH();
     }
   }
