@@ -73,259 +73,101 @@ __device__ __forceinline__ void wait_geq(const int* flag, int target, int* err, 
   __threadfence();
 }
 
-// One warp solves the c x c diagonal block for one right-hand side; lane l
-// holds rows l (v0) and 32 + l (v1).  Columns are taken eight at a time:
-// their eight current values are broadcast, every lane solves the 8 x 8
-// block redundantly, the owners take their rows' results and every lane
-// updates its rows beyond the block.  Each row receives exactly the updates
-// of column-by-column substitution, one FMA each, in the same column order,
-// so the result is the same to the bit; the dependent chain per column is one
-// FMA and one multiply instead of a shuffle round trip.
-__device__ __forceinline__ void diag_solve_fwd_warp(const double (*D)[kSnCols + 1], const double* rinv, double& v0,
-                                                    double& v1, int c) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k0 = 0; k0 < kSnCols; k0 += 8) {
-    if (k0 < c) {  // warp-uniform
-      double y[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = __shfl_sync(0xffffffffu, k0 < 32 ? v0 : v1, (k0 + i) & 31);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (k0 + i < c) {
-          double t = y[i];
-#pragma unroll
-          for (int j = 0; j < i; ++j) t -= D[k0 + i][k0 + j] * y[j];
-          y[i] = t * rinv[k0 + i];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (lane == ((k0 + i) & 31) && k0 + i < c) {
-          if (k0 < 32) v0 = y[i];
-          else v1 = y[i];
-        }
-      }
-      if (k0 < 32 && lane >= k0 + 8 && lane < c) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v0 -= D[lane][k0 + j] * y[j];
-      }
-      if (lane + 32 >= k0 + 8 && lane + 32 < c) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v1 -= D[lane + 32][k0 + j] * y[j];
-      }
-    }
-  }
-}
-// L^T x = z, columns from the last: the same blocking, eight at a time from
-// the top, every row updated in descending column order as in the
-// column-by-column substitution.
-__device__ __forceinline__ void diag_solve_bwd_warp(const double (*D)[kSnCols + 1], const double* rinv, double& v0,
-                                                    double& v1, int c) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k0 = kSnCols - 8; k0 >= 0; k0 -= 8) {
-    if (k0 < c) {  // warp-uniform
-      double x[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = __shfl_sync(0xffffffffu, k0 < 32 ? v0 : v1, (k0 + i) & 31);
-#pragma unroll
-      for (int i = 7; i >= 0; --i) {
-        if (k0 + i < c) {
-          double t = x[i];
-#pragma unroll
-          for (int j = 7; j > i; --j)
-            if (k0 + j < c) t -= D[k0 + j][k0 + i] * x[j];
-          x[i] = t * rinv[k0 + i];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (lane == ((k0 + i) & 31) && k0 + i < c) {
-          if (k0 < 32) v0 = x[i];
-          else v1 = x[i];
-        }
-      }
-      if (lane < k0 && lane < c) {
-#pragma unroll
-        for (int j = 7; j >= 0; --j)
-          if (k0 + j < c) v0 -= D[k0 + j][lane] * x[j];
-      }
-      if (k0 >= 32 && lane + 32 < k0 && lane + 32 < c) {
-#pragma unroll
-        for (int j = 7; j >= 0; --j)
-          if (k0 + j < c) v1 -= D[k0 + j][lane + 32] * x[j];
-      }
-    }
-  }
-}
-
-// The same blocking on the factor's scaled copy of the block: D holds the
+// Substitution with the factor's scaled copy of a diagonal block, by one warp:
+// lane l holds rows l (v0) and 32 + l (v1).  D (shared, row-major) holds the
 // unit lower triangle L_ij / L_ii below its diagonal.  Forward: L y = b is
 // D y = b / L_ii, so each unknown is its scaled right-hand side minus the
-// scaled products of the unknowns before it -- one FMA per column on the
-// dependent chain (FP64 latency is about 23 cycles on sm_100a, a shuffle
-// about 26), against an FMA and a multiply with the unscaled block.
-// Backward: L^T x = z is D^T w = z with w_i = L_ii x_i; the caller scales w.
-__device__ __forceinline__ void unit_solve_fwd_warp(const double (*D)[kSnCols + 1], double& v0, double& v1, int c) {
+// scaled products of the unknowns before it.  Backward: L^T x = z is D^T w = z
+// with w_i = L_ii x_i; the caller scales w.
+//
+// Eight columns at a time: the block's values go through shared memory to
+// every lane (a 64-bit shuffle issues in 11 cycles on sm_100a), every lane
+// solves the 8 x 8 block redundantly and updates its rows beyond it.  The
+// coefficients are loaded off the chain: the lane's own while the block's
+// values arrive and its triangle is solved, the next triangle during the
+// update.  The dependent chain is one FMA (9 cycles) per column, eight for the
+// rows of the next block, and the exchange.  Each row gets its FMAs in the
+// column order of column-by-column substitution: the same result to the bit.
+//
+// vs (64 doubles): the c right-hand sides on entry (scaled by the caller going
+// forward), the solution on return.  Rows from c up to the next multiple of
+// eight: any values going forward; going backward vs and the rows of D are
+// zero there.
+constexpr int kLdD = kSnCols + 1;  // rows and columns of the block without bank conflicts
+template <bool kForward>
+__device__ __forceinline__ void subst_warp(const double* D, double* vs, int c) {
   const int lane = threadIdx.x & 31;
+  double v0 = vs[lane], v1 = vs[lane + 32];
+  const int nb = (c + 7) / 8;
+  double t[28];  // the 8 x 8 block below its diagonal, row by row
+  auto load_t = [&](int k0) {
 #pragma unroll
-  for (int k0 = 0; k0 < kSnCols; k0 += 8) {
-    if (k0 < c) {  // warp-uniform
-      double y[8];
+    for (int i = 1; i < 8; ++i)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = __shfl_sync(0xffffffffu, k0 < 32 ? v0 : v1, (k0 + i) & 31);
+      for (int j = 0; j < i; ++j) t[i * (i - 1) / 2 + j] = D[(k0 + i) * kLdD + k0 + j];
+  };
+  load_t(8 * (kForward ? 0 : nb - 1));
+#pragma unroll 1
+  for (int b = 0; b < nb; ++b) {
+    const int k0 = 8 * (kForward ? b : nb - 1 - b);
+    double u0[8], u1[8], y[8];  // the lane's two rows (forward) or columns (backward) against the block's columns
 #pragma unroll
-      for (int i = 1; i < 8; ++i) {
-        if (k0 + i < c) {
+    for (int j = 0; j < 8; j += 2) {
+      const double2 p = *reinterpret_cast<const double2*>(vs + k0 + j);
+      y[j] = p.x;
+      y[j + 1] = p.y;
+    }
 #pragma unroll
-          for (int j = 0; j < i; ++j) y[i] -= D[k0 + i][k0 + j] * y[j];
-        }
-      }
+    for (int j = 0; j < 8; ++j) {
+      u0[j] = kForward ? D[lane * kLdD + k0 + j] : D[(k0 + j) * kLdD + lane];
+      u1[j] = kForward ? D[(lane + 32) * kLdD + k0 + j] : D[(k0 + j) * kLdD + lane + 32];
+    }
+    if (kForward) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (lane == ((k0 + i) & 31) && k0 + i < c) {
-          if (k0 < 32) v0 = y[i];
-          else v1 = y[i];
-        }
-      }
-      if (k0 < 32 && lane >= k0 + 8 && lane < c) {
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v0 -= D[lane][k0 + j] * y[j];
-      }
-      if (lane + 32 >= k0 + 8 && lane + 32 < c) {
+        for (int i = j + 1; i < 8; ++i) y[i] -= t[i * (i - 1) / 2 + j] * y[j];
+    } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v1 -= D[lane + 32][k0 + j] * y[j];
-      }
+      for (int j = 7; j >= 0; --j)
+#pragma unroll
+        for (int i = j - 1; i >= 0; --i) y[i] -= t[j * (j - 1) / 2 + i] * y[j];
+    }
+    const int k1 = kForward ? k0 + 8 : k0 - 8;  // the next block
+    if (b + 1 < nb) load_t(k1);
+    if (kForward ? lane >= k1 : lane < k0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v0 -= u0[kForward ? j : 7 - j] * y[kForward ? j : 7 - j];
+    }
+    if (kForward ? lane + 32 >= k1 : lane + 32 < k0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v1 -= u1[kForward ? j : 7 - j] * y[kForward ? j : 7 - j];
+    }
+    // the next block's values, and this block's solution
+    if (lane >= k1 && lane < k1 + 8) vs[lane] = v0;
+    if (lane + 32 >= k1 && lane + 32 < k1 + 8) vs[lane + 32] = v1;
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) *reinterpret_cast<double2*>(vs + k0 + j) = make_double2(y[j], y[j + 1]);
     }
   }
-}
-__device__ __forceinline__ void unit_solve_bwd_warp(const double (*D)[kSnCols + 1], double& v0, double& v1, int c) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k0 = kSnCols - 8; k0 >= 0; k0 -= 8) {
-    if (k0 < c) {  // warp-uniform
-      double x[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = __shfl_sync(0xffffffffu, k0 < 32 ? v0 : v1, (k0 + i) & 31);
-#pragma unroll
-      for (int i = 6; i >= 0; --i) {
-        if (k0 + i < c) {
-#pragma unroll
-          for (int j = 7; j > i; --j)
-            if (k0 + j < c) x[i] -= D[k0 + j][k0 + i] * x[j];
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (lane == ((k0 + i) & 31) && k0 + i < c) {
-          if (k0 < 32) v0 = x[i];
-          else v1 = x[i];
-        }
-      }
-      if (lane < k0 && lane < c) {
-#pragma unroll
-        for (int j = 7; j >= 0; --j)
-          if (k0 + j < c) v0 -= D[k0 + j][lane] * x[j];
-      }
-      if (k0 >= 32 && lane + 32 < k0 && lane + 32 < c) {
-#pragma unroll
-        for (int j = 7; j >= 0; --j)
-          if (k0 + j < c) v1 -= D[k0 + j][lane + 32] * x[j];
-      }
-    }
-  }
+  __syncwarp();
 }
 
-// Dense lower-triangular solve of the c x c diagonal block held in D (shared)
-// for nrhs columns of ys (row-major c x nrhs), forward (L y = b) or backward
-// (L^T x = z).  nrhs == 1 runs in one warp (the blocked substitution above).
-__device__ void diag_solve(const double (*D)[kSnCols + 1], const double* rinv, double* ys, int c, int nrhs,
-                           bool forward, bool scaled = false) {
-  const int tid = threadIdx.x;
-  if (nrhs == 1 && scaled) {  // D: the factor's scaled copy; rinv: 1 / L_ii
-    if (tid < 32) {
-      const int lane = tid;
-      double v0 = lane < c ? ys[lane] : 0.0;
-      double v1 = lane + 32 < c ? ys[lane + 32] : 0.0;
-      if (forward) {
-        v0 *= lane < c ? rinv[lane] : 0.0;
-        v1 *= lane + 32 < c ? rinv[lane + 32] : 0.0;
-        unit_solve_fwd_warp(D, v0, v1, c);
-      } else {
-        unit_solve_bwd_warp(D, v0, v1, c);
-        v0 *= lane < c ? rinv[lane] : 0.0;
-        v1 *= lane + 32 < c ? rinv[lane + 32] : 0.0;
-      }
-      if (lane < c) ys[lane] = v0;
-      if (lane + 32 < c) ys[lane + 32] = v1;
-    }
-    __syncthreads();
-    return;
-  }
-  if (nrhs == 1) {
-    if (tid < 32) {
-      const int lane = tid;
-      double v0 = lane < c ? ys[lane] : 0.0;
-      double v1 = lane + 32 < c ? ys[lane + 32] : 0.0;
-      if (forward) diag_solve_fwd_warp(D, rinv, v0, v1, c);
-      else diag_solve_bwd_warp(D, rinv, v0, v1, c);
-      if (lane < c) ys[lane] = v0;
-      if (lane + 32 < c) ys[lane + 32] = v1;
-    }
-    __syncthreads();
-    return;
-  }
-  if (forward) {
-    for (int j = 0; j < c; ++j) {
-      for (int col = tid; col < nrhs; col += blockDim.x) ys[j * nrhs + col] *= rinv[j];
-      __syncthreads();
-      for (int idx = tid; idx < (c - j - 1) * nrhs; idx += blockDim.x) {
-        const int k = j + 1 + idx / nrhs, col = idx % nrhs;
-        ys[k * nrhs + col] -= D[k][j] * ys[j * nrhs + col];
-      }
-      __syncthreads();
-    }
-  } else {
-    for (int j = c - 1; j >= 0; --j) {
-      for (int col = tid; col < nrhs; col += blockDim.x) ys[j * nrhs + col] *= rinv[j];
-      __syncthreads();
-      for (int idx = tid; idx < j * nrhs; idx += blockDim.x) {
-        const int k = idx / nrhs, col = idx % nrhs;
-        ys[k * nrhs + col] -= D[j][k] * ys[j * nrhs + col];
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// Lower triangle of the diagonal block into D with asynchronous copies
-// (issued before a dependency wait; coalesced per column), and the
-// reciprocals of its diagonal once the copies have landed.
-__device__ __forceinline__ void load_diag_start(double (*D)[kSnCols + 1], const double* P, int c, int64_t ld) {
+// Lower triangle of a diagonal block's scaled copy Q (c x c, column-major)
+// into D (row-major) with asynchronous copies, issued before a dependency
+// wait.
+__device__ __forceinline__ void load_diag_scaled(double* D, const double* Q, int c) {
   for (int idx = threadIdx.x; idx < c * c; idx += blockDim.x) {
     const int j = idx / c, i = idx - j * c;
-    if (i >= j) cp_async8(&D[i][j], P + (int64_t)j * ld + i);
+    if (i >= j) cp_async8(&D[i * kLdD + j], Q + idx);
   }
 }
-__device__ __forceinline__ void load_diag_finish(double (*D)[kSnCols + 1], double* rinv, int c, bool scaled = false) {
-  cp_async_wait_all();
-  __syncthreads();
-  if ((int)threadIdx.x < c) rinv[threadIdx.x] = scaled ? D[threadIdx.x][threadIdx.x] : 1.0 / D[threadIdx.x][threadIdx.x];
-  __syncthreads();
-}
-// the factor's scaled copy of the block (c x c, column-major), lower triangle
-__device__ __forceinline__ void load_diag_start_scaled(double (*D)[kSnCols + 1], const double* Q, int c) {
-  for (int idx = threadIdx.x; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx - j * c;
-    if (i >= j) cp_async8(&D[i][j], Q + idx);
-  }
-}
-// single column: the scaled copy when the view has one, else the panel's block
-__device__ __forceinline__ void load_diag_start_1(double (*D)[kSnCols + 1], const SweepView& V, const double* Lb, int s,
-                                                  const double* P, int c, int64_t ld) {
-  if (V.Dptr) load_diag_start_scaled(D, Lb + V.Dptr[s], c);
-  else load_diag_start(D, P, c, ld);
+// rows c .. up to the next multiple of eight: zero (the backward substitution reads them)
+__device__ __forceinline__ void zero_diag_tail(double* D, int c) {
+  for (int idx = threadIdx.x; idx < ((8 - c % 8) % 8) * kSnCols; idx += blockDim.x)
+    D[(c + idx / kSnCols) * kLdD + idx % kSnCols] = 0.0;
 }
 
 // Row-chunk products, single right-hand side.  The panel values are loaded
@@ -494,75 +336,24 @@ __device__ __forceinline__ int next_task(const SweepView& V, int* counter, bool 
 //     ready counter of each supernode owning one of the rows;
 //   chunk task (s, r0..r1), r0 >= 128: wait for y_s, push the same way.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double* Lb, int nrhs, int* err,
-                                         double (*D)[kSnCols + 1], double* rinv, double* ys,
-                                         unsigned long long* stamp = nullptr) {
+// Shared memory of the single-column tasks.
+struct TaskSmem {
+  double D[kSnCols * kLdD];
+  double rows[kSnCols][32];  // forward diagonal task: the chunk rows of warp 0, which runs the substitution
+  double ys[kSnCols];        // y_s going forward; z, then x_s going backward
+  double seg[4][kSnCols];    // backward: per warp, the column sums over its rows
+};
+
+// The chunk's pushes and counts, after y_s is in ys: shared by both kinds of
+// forward task.
+__device__ __forceinline__ void fwd_publish(const SweepView& V, const SolveTask& T, int t, int64_t r, int tg_o, int tg_d,
+                                            int tg_ex) {
   int* ready = V.sync;
-  int* ydone = V.sync + V.nsn;
-  double* x = V.x;
   const int tid = threadIdx.x;
-  const SolveTask T = V.tasks[t];
-  const int s = T.s;
-  const int f = V.sn_first[s];
-  const int c = V.sn_first[s + 1] - f;
-  const int64_t rp = V.rows_ptr[s];
-  const int64_t r = V.rows_ptr[s + 1] - rp;
-  const int64_t ld = c + r;
-  const double* P = Lb + V.Lptr[s];
-  const double* Pc = P + c;
-  const int i = T.r0 + tid;
-  const bool row_on = i < T.r1;
-  FwdRegs R;
-  if (nrhs == 1) pre_fwd(R, Pc, c, ld, i, row_on);
-  const int row_i = row_on ? V.sn_rows[rp + i] : 0;  // the row this thread pushes to (read before the wait)
-  const bool queued = in_queue(V, t);
-  // this thread's target supernode with its diagonal task and input count,
-  // read before the wait (a chunk of at most blockDim rows feeds at most
-  // blockDim supernodes: one entry per thread)
-  int tg_o = -1, tg_d = -1, tg_ex = 0;
-  if (V.queue && T.r1 > T.r0) {
-    const int k = V.tgt_ptr[t] + tid;
-    if (k < V.tgt_ptr[t + 1]) {
-      tg_o = V.tgt[k];
-      tg_d = V.diag_task[tg_o];
-      tg_ex = V.expect[tg_o];
-    }
-  }
-  const bool sc = nrhs == 1 && V.Dptr != nullptr;
-  if (T.kind == 0) {
-    if (sc) load_diag_start_scaled(D, Lb + V.Dptr[s], c);
-    else load_diag_start(D, P, c, ld);
-    if (tid == 0 && !queued) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
-    __syncthreads();
-    if (stamp && tid == 0) *stamp = gtime();
-    for (int idx = tid; idx < c * nrhs; idx += blockDim.x) ys[idx] = __ldcg(x + (int64_t)f * nrhs + idx);
-    load_diag_finish(D, rinv, c, sc);
-    diag_solve(D, rinv, ys, c, nrhs, true, sc);
-    for (int idx = tid; idx < c * nrhs; idx += blockDim.x) x[(int64_t)f * nrhs + idx] = ys[idx];
-    // y_s is published together with the first chunk's pushes below: one fence for both
-  } else {
-    if (tid == 0 && !queued) wait_geq(ydone + s, 1, err, 2, spin_limit(V));
-    __syncthreads();
-    if (stamp && tid == 0) *stamp = gtime();
-    for (int idx = tid; idx < c * nrhs; idx += blockDim.x) ys[idx] = __ldcg(x + (int64_t)f * nrhs + idx);
-    __syncthreads();
-  }
-  if (T.r1 > T.r0) {
-    if (nrhs == 1) {
-      if (row_on) atomicAdd(x + row_i, -fin_fwd(R, ys, c));
-    } else if (row_on) {
-      double* dst = x + (int64_t)row_i * nrhs;
-      for (int col = 0; col < nrhs; ++col) {
-        double a = 0.0;
-        for (int j = 0; j < c; ++j) a += __ldg(Pc + (int64_t)j * ld + i) * ys[j * nrhs + col];
-        atomicAdd(dst + col, -a);
-      }
-    }
-  }
   __threadfence();
   __syncthreads();
   if (T.kind == 0) {
-    if (tid == 0) atomicExch(ydone + s, 1);
+    if (tid == 0) atomicExch(V.sync + V.nsn + T.s, 1);
     if (V.queue) {  // y_s is out: the other row chunks of s are ready (they follow this task)
       const int nx = max(1, (int)((r + kChunkRows - 1) / kChunkRows)) - 1;
       for (int k = tid; k < nx; k += blockDim.x) q_push(V, t + 1 + k);
@@ -581,29 +372,97 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
   }
 }
 
-__global__ void __launch_bounds__(kSolveThreads) k_fwd_persistent(
-    int ntask, const SolveTask* __restrict__ tasks, const int* __restrict__ sn_first,
-    const int64_t* __restrict__ rows_ptr, const int* __restrict__ sn_rows, const int64_t* __restrict__ Lptr,
-    double* const* Lbase, double* x, int nrhs, const int* __restrict__ tgt_ptr, const int* __restrict__ tgt,
-    const int* __restrict__ expect, int* sync, int nsn, int* err) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  extern __shared__ double ys[];  // c x nrhs
+__device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M,
+                                         unsigned long long* stamp = nullptr) {
+  int* ready = V.sync;
+  int* ydone = V.sync + V.nsn;
+  double* x = V.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const SolveTask T = V.tasks[t];
+  const int s = T.s;
+  const int f = V.sn_first[s];
+  const int c = V.sn_first[s + 1] - f;
+  const int64_t rp = V.rows_ptr[s];
+  const int64_t r = V.rows_ptr[s + 1] - rp;
+  const int64_t ld = c + r;
+  const double* Pc = Lb + V.Lptr[s] + c;
+  const int i = T.r0 + tid;
+  const bool row_on = i < T.r1;
+  const int row_i = row_on ? V.sn_rows[rp + i] : 0;  // the row this thread pushes to (read before the wait)
+  const bool queued = in_queue(V, t);
+  // this thread's target supernode with its diagonal task and input count,
+  // read before the wait (a chunk of at most blockDim rows feeds at most
+  // blockDim supernodes: one entry per thread)
+  int tg_o = -1, tg_d = -1, tg_ex = 0;
+  if (V.queue && T.r1 > T.r0) {
+    const int k = V.tgt_ptr[t] + tid;
+    if (k < V.tgt_ptr[t + 1]) {
+      tg_o = V.tgt[k];
+      tg_d = V.diag_task[tg_o];
+      tg_ex = V.expect[tg_o];
+    }
+  }
+  if (T.kind == 0 && tid < 32) {
+    // Warp 0 substitutes: its registers hold coefficients, so its share of
+    // the first chunk waits in shared memory.
+    load_diag_scaled(M.D, Lb + V.Dptr[s], c);
+    if (row_on)
+      for (int j = 0; j < c; ++j) cp_async8(&M.rows[j][lane], Pc + (int64_t)j * ld + i);
+    cp_async_wait_all();
+    __syncthreads();
+    if (lane == 0 && !queued) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
+    __syncwarp();
+    if (stamp && lane == 0) *stamp = gtime();
+    const double x0 = lane < c ? __ldcg(x + f + lane) : 0.0;
+    const double x1 = lane + 32 < c ? __ldcg(x + f + 32 + lane) : 0.0;
+    M.ys[lane] = lane < c ? x0 * M.D[lane * kLdD + lane] : 0.0;  // the copy's diagonal: 1 / L_ii
+    M.ys[lane + 32] = lane + 32 < c ? x1 * M.D[(lane + 32) * kLdD + lane + 32] : 0.0;
+    __syncwarp();
+    subst_warp<true>(M.D, M.ys, c);
+    if (lane < c) x[f + lane] = M.ys[lane];
+    if (lane + 32 < c) x[f + 32 + lane] = M.ys[lane + 32];
+    // y_s is published together with the first chunk's pushes below: one fence for both
+    __syncthreads();
+    if (row_on) {
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+      for (int j = 0; j < kSnCols; j += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] += (j + u < c ? M.rows[j + u][lane] : 0.0) * (j + u < c ? M.ys[j + u] : 0.0);
+      atomicAdd(x + row_i, -((a[0] + a[1]) + (a[2] + a[3])));
+    }
+  } else {
+    FwdRegs R;
+    pre_fwd(R, Pc, c, ld, i, row_on);
+    if (T.kind == 0) {
+      load_diag_scaled(M.D, Lb + V.Dptr[s], c);
+      cp_async_wait_all();
+      __syncthreads();
+    } else {
+      if (tid == 0 && !queued) wait_geq(ydone + s, 1, err, 2, spin_limit(V));
+      __syncthreads();
+      if (stamp && tid == 0) *stamp = gtime();
+      if (tid < c) M.ys[tid] = __ldcg(x + f + tid);
+    }
+    __syncthreads();
+    if (row_on) atomicAdd(x + row_i, -fin_fwd(R, M.ys, c));
+  }
+  fwd_publish(V, T, t, r, tg_o, tg_d, tg_ex);
+}
+
+// All tasks claimed in schedule order (no queue): the allocation-free solve.
+__global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_persistent(const SweepView V, int* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   __shared__ int task_id;
-  int* counter = sync + 4 * nsn;
-  const SweepView V{tasks, sn_first, rows_ptr, sn_rows, Lptr, Lbase, x, tgt_ptr, tgt, expect,
-                    nullptr, nullptr, nullptr, sync, nsn, ntask};
-  const double* Lb = *Lbase;
+  const double* Lb = *V.Lbase;
   for (;;) {
-    if (threadIdx.x == 0) task_id = atomicAdd(counter, 1);
+    if (threadIdx.x == 0) task_id = atomicAdd(V.sync + 4 * V.nsn, 1);
     __syncthreads();
     const int t = task_id;
     __syncthreads();
-    if (t >= ntask) break;
-    unsigned long long* rec = g_timeline_f ? g_timeline_f + 4 * (size_t)t : nullptr;
-    if (rec && threadIdx.x == 0) rec[0] = gtime();
-    fwd_task(V, t, Lb, nrhs, err, D, rinv, ys, rec ? rec + 1 : nullptr);
-    if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
+    if (t >= V.ntask) break;
+    fwd_task(V, t, Lb, err, M);
   }
 }
 
@@ -616,13 +475,12 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_persistent(
 //     the owners of the first chunk's rows, z = y_s - partials (fixed order,
 //     so the backward sweep is deterministic), solve with L11^T, publish x_s.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double* Lb, int nrhs, int* err,
-                                         double (*D)[kSnCols + 1], double* rinv, double (*seg)[kSnCols],
-                                         double* zs, unsigned long long* stamp = nullptr) {
+__device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M,
+                                         unsigned long long* stamp = nullptr) {
   int* cdone = V.sync + 2 * V.nsn;
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x;
   const SolveTask T = V.tasks[t];
   const int s = T.s;
   const int f = V.sn_first[s];
@@ -633,23 +491,23 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   const double* P = Lb + V.Lptr[s];
   const int nr = T.r1 - T.r0;
   FwdRegs R;
-  if (nrhs == 1 && nr > 0) pre_fwd(R, P + c, c, ld, T.r0 + tid, tid < nr);
-  // one chunk row per thread for a single column: its index read before the wait
-  const int row_t = (nrhs == 1 && tid < nr) ? V.sn_rows[rp + T.r0 + tid] : 0;
-  const bool sc = nrhs == 1 && V.Dptr != nullptr;
+  if (nr > 0) pre_fwd(R, P + c, c, ld, T.r0 + tid, tid < nr);
+  // one chunk row per thread: its index read before the wait
+  const int row_t = tid < nr ? V.sn_rows[rp + T.r0 + tid] : 0;
   if (T.kind == 0) {
-    if (sc) load_diag_start_scaled(D, Lb + V.Dptr[s], c);
-    else load_diag_start(D, P, c, ld);
+    load_diag_scaled(M.D, Lb + V.Dptr[s], c);
+    zero_diag_tail(M.D, c);
   }
   const bool queued = in_queue(V, t);
-  // Diagonal task, one column: y_s (written by the forward sweep only) is read
-  // before any wait, and the column sums of the other chunks once their count
-  // is complete, while the owner of the first chunk's rows is still awaited
-  // (on the top chain that owner is the block just above, finished last).
-  const bool pre = T.kind == 0 && nrhs == 1 && V.bacc != nullptr;
+  // Diagonal task: y_s (written by the forward sweep only) is read before any
+  // wait, and with one accumulator per column the sums of the other chunks
+  // once their count is complete, while the owner of the first chunk's rows
+  // is still awaited (on the top chain that owner is the block just above,
+  // finished last).
+  const bool pre = T.kind == 0 && V.bacc != nullptr;
   const bool more = V.nchunk[s] > 1;
   double y_pre = 0.0, acc_pre = 0.0;
-  if (pre && tid < c) y_pre = __ldcg(x + f + tid);
+  if (T.kind == 0 && tid < c) y_pre = __ldcg(x + f + tid);
   // the chunk's rows need their owners' x; the diagonal task also its other chunks
   if (!queued) {  // one polling thread per owner (and one for the chunk count)
     const int q0 = V.tgt_ptr[t], nq = V.tgt_ptr[t + 1] - q0;
@@ -666,37 +524,16 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   }
   __syncthreads();
   if (stamp && tid == 0) *stamp = gtime();
-  double* zx = zs + (T.kind == 0 ? kSnCols * nrhs : 0);  // chunk rows live after the diagonal block
-  if (nr > 0) {
-    if (nrhs == 1) {  // nr <= blockDim.x: one row per thread
-      bwd_row_sums(R, tid < nr ? __ldcg(x + row_t) : 0.0, seg);
-    } else {
-      for (int idx = tid; idx < nr * nrhs; idx += blockDim.x) {
-        const int ii = idx / nrhs, col = idx % nrhs;
-        zx[idx] = __ldcg(x + (int64_t)V.sn_rows[rp + T.r0 + ii] * nrhs + col);
-      }
-    }
+  if (nr > 0) {  // nr <= blockDim.x: one row per thread
+    bwd_row_sums(R, tid < nr ? __ldcg(x + row_t) : 0.0, M.seg);
     __syncthreads();
   }
   if (T.kind == 1) {
-    const int chunk = T.r0 / kChunkRows;
-    double* pp = V.part + (V.part_off[s] + (int64_t)chunk * c) * nrhs;
-    if (nrhs == 1 && V.bacc) {  // one accumulator per column: the diagonal task reads c values
-      for (int j = tid; j < c; j += blockDim.x)
-        atomicAdd(V.bacc + f + j, (seg[0][j] + seg[1][j]) + (seg[2][j] + seg[3][j]));
-    } else if (nrhs == 1) {
-      for (int j = tid; j < c; j += blockDim.x) pp[j] = (seg[0][j] + seg[1][j]) + (seg[2][j] + seg[3][j]);
-    } else {
-      for (int j = warp; j < c; j += nw) {
-        const double* colp = P + (int64_t)j * ld + c + T.r0;
-        for (int col = 0; col < nrhs; ++col) {
-          double acc = 0.0;
-          for (int ii = lane; ii < nr; ii += 32) acc += __ldg(colp + ii) * zx[ii * nrhs + col];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          if (lane == 0) pp[j * nrhs + col] = acc;
-        }
-      }
+    const int j = tid;
+    if (j < c) {
+      const double v = (M.seg[0][j] + M.seg[1][j]) + (M.seg[2][j] + M.seg[3][j]);
+      if (V.bacc) atomicAdd(V.bacc + f + j, v);  // one accumulator per column: the diagonal task reads c values
+      else V.part[V.part_off[s] + (int64_t)(T.r0 / kChunkRows) * c + j] = v;
     }
     __threadfence();
     __syncthreads();
@@ -708,60 +545,44 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
       }
     }
   } else {
-    // z = y_s - (first chunk, computed here) - (other chunks, in order)
-    const int nch = V.nchunk[s];
-    const double* pp = V.part + V.part_off[s] * nrhs;
-    if (nrhs == 1) {
-      // the other chunks' partials: thread (j, h) sums chunks q = 1 + h, 3 + h, ...
-      // with eight loads in flight; fixed order, so still deterministic
-      double* psum = zx;  // the chunk rows are consumed: reuse as [2][64]
-      if (pre) {  // y_s and the column sums are in registers (c <= blockDim.x)
-        if (tid < c) {
-          double v = y_pre;
-          if (nr > 0) v -= (seg[0][tid] + seg[1][tid]) + (seg[2][tid] + seg[3][tid]);
-          if (more) v -= acc_pre;
-          zs[tid] = v;
-        }
-      } else if (nch > 1) {
-        const int j = tid & (kSnCols - 1), h = tid / kSnCols;
-        double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (j < c && h < 2) {
-          int q = 1 + h;
-          for (; q + 14 < nch; q += 16) {
+    // z = y_s - (first chunk, computed here) - (other chunks)
+    if (!pre && more) {
+      // without accumulators: thread (j, h) sums the partials of chunks q = 1 + h, 3 + h, ...
+      // with eight loads in flight; fixed order
+      const int nch = V.nchunk[s];
+      const double* pp = V.part + V.part_off[s];
+      const int j = tid & (kSnCols - 1), h = tid / kSnCols;
+      double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (j < c) {
+        int q = 1 + h;
+        for (; q + 14 < nch; q += 16) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] += __ldcg(pp + (int64_t)(q + 2 * u) * c + j);
-          }
+          for (int u = 0; u < 8; ++u) a[u] += __ldcg(pp + (int64_t)(q + 2 * u) * c + j);
+        }
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (q + 2 * u < nch) a[u] += __ldcg(pp + (int64_t)(q + 2 * u) * c + j);
-        }
-        if (h < 2) psum[h * kSnCols + j] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-        __syncthreads();
+        for (int u = 0; u < 8; ++u)
+          if (q + 2 * u < nch) a[u] += __ldcg(pp + (int64_t)(q + 2 * u) * c + j);
       }
-      if (!pre) {
-        for (int j = tid; j < c; j += blockDim.x) {
-          double v = __ldcg(x + f + j);
-          if (nr > 0) v -= (seg[0][j] + seg[1][j]) + (seg[2][j] + seg[3][j]);
-          if (nch > 1) v -= psum[j] + psum[kSnCols + j];
-          zs[j] = v;
-        }
-      }
-    } else {
-      for (int idx = tid; idx < c * nrhs; idx += blockDim.x) {
-        const int j = idx / nrhs, col = idx % nrhs;
-        double v = __ldcg(x + (int64_t)f * nrhs + idx);
-        if (nr > 0) {
-          double a = 0.0;
-          for (int ii = 0; ii < nr; ++ii) a += __ldg(P + (int64_t)j * ld + c + ii) * zx[ii * nrhs + col];
-          v -= a;
-        }
-        for (int q = 1; q < nch; ++q) v -= __ldcg(pp + (int64_t)q * c * nrhs + idx);
-        zs[idx] = v;
-      }
+      double* psum = &M.rows[0][0];  // free going backward
+      psum[h * kSnCols + j] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+      __syncthreads();
+      acc_pre = psum[j] + psum[kSnCols + j];
     }
-    load_diag_finish(D, rinv, c, sc);
-    diag_solve(D, rinv, zs, c, nrhs, false, sc);
-    for (int idx = tid; idx < c * nrhs; idx += blockDim.x) x[(int64_t)f * nrhs + idx] = zs[idx];
+    if (tid < kSnCols) {
+      double v = 0.0;
+      if (tid < c) {
+        v = y_pre;
+        if (nr > 0) v -= (M.seg[0][tid] + M.seg[1][tid]) + (M.seg[2][tid] + M.seg[3][tid]);
+        if (more) v -= acc_pre;
+      }
+      M.ys[tid] = v;
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if (tid < 32) {
+      subst_warp<false>(M.D, M.ys, c);
+      for (int j = tid; j < c; j += 32) x[f + j] = M.ys[j] * M.D[j * kLdD + j];
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0) atomicExch(xdone + s, 1);
@@ -769,31 +590,18 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   }
 }
 
-__global__ void __launch_bounds__(kSolveThreads) k_bwd_persistent(
-    int ntask, const SolveTask* __restrict__ tasks, const int* __restrict__ sn_first,
-    const int64_t* __restrict__ rows_ptr, const int* __restrict__ sn_rows, const int64_t* __restrict__ Lptr,
-    double* const* Lbase, double* x, int nrhs, const int* __restrict__ own_ptr, const int* __restrict__ own,
-    const int* __restrict__ nchunk, const int64_t* __restrict__ part_off, double* part, int* sync, int nsn,
-    int* err) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  __shared__ double seg[4][kSnCols];
-  extern __shared__ double zs[];  // max(c, chunk rows) x nrhs
+__global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_persistent(const SweepView V, int* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   __shared__ int task_id;
-  int* counter = sync + 4 * nsn + 1;
-  const SweepView V{tasks, sn_first, rows_ptr, sn_rows, Lptr, Lbase, x, own_ptr, own, nullptr,
-                    nchunk, part_off, part, sync, nsn, ntask};
-  const double* Lb = *Lbase;
+  const double* Lb = *V.Lbase;
   for (;;) {
-    if (threadIdx.x == 0) task_id = atomicAdd(counter, 1);
+    if (threadIdx.x == 0) task_id = atomicAdd(V.sync + 4 * V.nsn + 1, 1);
     __syncthreads();
     const int t = task_id;
     __syncthreads();
-    if (t >= ntask) break;
-    unsigned long long* rec = g_timeline_b ? g_timeline_b + 4 * (size_t)t : nullptr;
-    if (rec && threadIdx.x == 0) rec[0] = gtime();
-    bwd_task(V, t, Lb, nrhs, err, D, rinv, seg, zs, rec ? rec + 1 : nullptr);
-    if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
+    if (t >= V.ntask) break;
+    bwd_task(V, t, Lb, err, M);
   }
 }
 
@@ -823,8 +631,7 @@ constexpr int kMaxLeaders = 24;
 
 __device__ __forceinline__ int leader_blocks(const SolveTask& T) { return T.kind >> 4; }
 
-__device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err, double (*D)[kSnCols + 1],
-                           double* rinv, double* ys, double* ring) {
+__device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M, double* ring) {
   int* ready = V.sync;
   int* ydone = V.sync + V.nsn;
   double* x = V.x;
@@ -839,9 +646,8 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
     const int64_t r = V.rows_ptr[a + 1] - V.rows_ptr[a], ld = c + r;
     const double* P = Lb + V.Lptr[a];
     pre_fwd(R, P + c, c, ld, tid, tid < (r < kChunkRows ? r : (int64_t)kChunkRows));
-    load_diag_start_1(D, V, Lb, a, P, c, ld);
+    load_diag_scaled(M.D, Lb + V.Dptr[a], c);
   }
-  const bool sc = V.Dptr != nullptr;
   for (int q = a; q <= e; ++q) {
     const int f = V.sn_first[q], c = V.sn_first[q + 1] - f;
     const int64_t rp = V.rows_ptr[q], r = V.rows_ptr[q + 1] - rp;
@@ -851,14 +657,20 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
     __syncthreads();
     for (int j = tid; j < c; j += blockDim.x) {
       const int slot = (f + j - f_run) & (kRing - 1);
-      ys[j] = __ldcg(x + f + j) + ring[slot];  // the ring holds the negated in-run contributions
+      M.ys[j] = __ldcg(x + f + j) + ring[slot];  // the ring holds the negated in-run contributions
       ring[slot] = 0.0;
     }
-    load_diag_finish(D, rinv, c, sc);
-    diag_solve(D, rinv, ys, c, 1, true, sc);
-    for (int j = tid; j < c; j += blockDim.x) x[f + j] = ys[j];
+    cp_async_wait_all();
+    __syncthreads();
+    if (tid < 32) {
+      for (int j = tid; j < kSnCols; j += 32) M.ys[j] = j < c ? M.ys[j] * M.D[j * kLdD + j] : 0.0;
+      __syncwarp();
+      subst_warp<true>(M.D, M.ys, c);
+    }
+    __syncthreads();
+    for (int j = tid; j < c; j += blockDim.x) x[f + j] = M.ys[j];
     if (tid < r1) {
-      const double v = fin_fwd(R, ys, c);
+      const double v = fin_fwd(R, M.ys, c);
       const int row = V.sn_rows[rp + tid];
       if (row < f_end) ring[(row - f_run) & (kRing - 1)] -= v;  // inside the run: one writer per row
       else atomicAdd(x + row, -v);
@@ -876,13 +688,13 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
       const int64_t rn = V.rows_ptr[q + 2] - V.rows_ptr[q + 1], ldn = cn + rn;
       const double* Pn = Lb + V.Lptr[q + 1];
       pre_fwd(R, Pn + cn, cn, ldn, tid, tid < (rn < kChunkRows ? rn : (int64_t)kChunkRows));
-      load_diag_start_1(D, V, Lb, q + 1, Pn, cn, ldn);
+      load_diag_scaled(M.D, Lb + V.Dptr[q + 1], cn);
     }
   }
 }
 
-__device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err, double (*D)[kSnCols + 1],
-                           double* rinv, double (*seg)[kSnCols], double* zs, double* ring) {
+__device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M, double* ring) {
+  double (*seg)[kSnCols] = M.seg;
   int* cdone = V.sync + 2 * V.nsn;
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
@@ -897,9 +709,9 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
     const double* P = Lb + V.Lptr[e];
     const int r1 = (int)(r < kChunkRows ? r : (int64_t)kChunkRows);
     if (r1 > 0) pre_fwd(R, P + c, c, ld, tid, tid < r1);
-    load_diag_start_1(D, V, Lb, e, P, c, ld);
+    load_diag_scaled(M.D, Lb + V.Dptr[e], c);
+    zero_diag_tail(M.D, c);
   }
-  const bool sc = V.Dptr != nullptr;
   for (int q = e; q >= a; --q) {
     const int f = V.sn_first[q], c = V.sn_first[q + 1] - f;
     const int64_t rp = V.rows_ptr[q], r = V.rows_ptr[q + 1] - rp;
@@ -912,7 +724,6 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
       if (tid == blockDim.x - 1) wait_geq(cdone + q, V.nchunk[q] - (r1 > 0 ? 1 : 0), err, 4, spin_limit(V));
     }
     __syncthreads();
-    double* zx = zs + kSnCols;
     if (r1 > 0) {
       double zi = 0.0;
       if (tid < r1) {
@@ -925,7 +736,7 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
     // z = y_q - (first chunk) - (other chunks, fixed order)
     const int nch = V.nchunk[q];
     const double* pp = V.part + V.part_off[q];
-    double* psum = zx;  // the chunk rows are consumed: reuse as [2][64]
+    double* psum = &M.rows[0][0];  // [2][64]
     if (nch > 1 && V.bacc) {
       for (int j = tid; j < c; j += blockDim.x) {
         psum[j] = __ldcg(V.bacc + f + j);
@@ -952,13 +763,17 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
       double v = __ldcg(x + f + j);
       if (r1 > 0) v -= (seg[0][j] + seg[1][j]) + (seg[2][j] + seg[3][j]);
       if (nch > 1) v -= psum[j] + psum[kSnCols + j];
-      zs[j] = v;
+      M.ys[j] = v;
     }
-    load_diag_finish(D, rinv, c, sc);
-    diag_solve(D, rinv, zs, c, 1, false, sc);
+    if (tid >= c && tid < kSnCols) M.ys[tid] = 0.0;
+    cp_async_wait_all();
+    __syncthreads();
+    if (tid < 32) subst_warp<false>(M.D, M.ys, c);
+    __syncthreads();
     for (int j = tid; j < c; j += blockDim.x) {
-      x[f + j] = zs[j];
-      ring[(f + j - f_run) & (kRing - 1)] = zs[j];
+      const double v = M.ys[j] * M.D[j * kLdD + j];
+      x[f + j] = v;
+      ring[(f + j - f_run) & (kRing - 1)] = v;
     }
     __threadfence();
     __syncthreads();
@@ -970,7 +785,8 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
       const double* Pn = Lb + V.Lptr[q - 1];
       const int r1n = (int)(rn < kChunkRows ? rn : (int64_t)kChunkRows);
       if (r1n > 0) pre_fwd(R, Pn + cn, cn, ldn, tid, tid < r1n);
-      load_diag_start_1(D, V, Lb, q - 1, Pn, cn, ldn);
+      load_diag_scaled(M.D, Lb + V.Dptr[q - 1], cn);
+      zero_diag_tail(M.D, cn);
     }
   }
 }
@@ -981,10 +797,9 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
 // (168 registers) for both sweeps; the backward with leaders two.
 template <bool kLeaders>
 __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView V, int* err) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  __shared__ double ys[kSnCols];
-  __shared__ double ring[kRing];
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
+  __shared__ double ring[kLeaders ? kRing : 1];
   __shared__ int task_id;
   const double* Lb = *V.Lbase;
   int phase = 0;
@@ -995,9 +810,9 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView
     if (rec && threadIdx.x == 0) rec[0] = gtime();
     if (kLeaders && (V.tasks[t].kind & 15) == 3) {
       if (rec && threadIdx.x == 0) rec[1] = gtime();
-      fwd_leader(V, t, Lb, err, D, rinv, ys, ring);
+      fwd_leader(V, t, Lb, err, M, ring);
     } else {
-      fwd_task(V, t, Lb, 1, err, D, rinv, ys, rec ? rec + 1 : nullptr);
+      fwd_task(V, t, Lb, err, M, rec ? rec + 1 : nullptr);
     }
     if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
   }
@@ -1005,11 +820,9 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView
 
 template <bool kLeaders>
 __global__ void __launch_bounds__(kSolveThreads, kLeaders ? 2 : 3) k_bwd_queued(const SweepView V, int* err) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  __shared__ double seg[4][kSnCols];
-  __shared__ double zs[kSnCols + kChunkRows];
-  __shared__ double ring[kRing];
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
+  __shared__ double ring[kLeaders ? kRing : 1];
   __shared__ int task_id;
   const double* Lb = *V.Lbase;
   int phase = 0;
@@ -1020,9 +833,9 @@ __global__ void __launch_bounds__(kSolveThreads, kLeaders ? 2 : 3) k_bwd_queued(
     if (rec && threadIdx.x == 0) rec[0] = gtime();
     if (kLeaders && (V.tasks[t].kind & 15) == 3) {
       if (rec && threadIdx.x == 0) rec[1] = gtime();
-      bwd_leader(V, t, Lb, err, D, rinv, seg, zs, ring);
+      bwd_leader(V, t, Lb, err, M, ring);
     } else {
-      bwd_task(V, t, Lb, 1, err, D, rinv, seg, zs, rec ? rec + 1 : nullptr);
+      bwd_task(V, t, Lb, err, M, rec ? rec + 1 : nullptr);
     }
     if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
   }
@@ -1325,9 +1138,8 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_models(int nstatic, co
                                                                   const SweepView* __restrict__ views,
                                                                   const int* __restrict__ active, int* counter,
                                                                   int* err, int qlim) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  __shared__ double ys[kSnCols];
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   __shared__ int2 mt_sh;
   const SweepView& V0 = views[0];  // the shared queue lives in every view
   int phase = 0;
@@ -1336,7 +1148,7 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_models(int nstatic, co
                                     &mt_sh, spin_limit(V0));
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
-    fwd_task(V, mt.y, *V.Lbase, 1, err, D, rinv, ys);
+    fwd_task(V, mt.y, *V.Lbase, err, M);
   }
 }
 
@@ -1344,10 +1156,8 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
                                                                   const SweepView* __restrict__ views,
                                                                   const int* __restrict__ active, int* counter,
                                                                   int* err, int qlim) {
-  __shared__ double D[kSnCols][kSnCols + 1];
-  __shared__ double rinv[kSnCols];
-  __shared__ double seg[4][kSnCols];
-  __shared__ double zs[kSnCols + kChunkRows];
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   __shared__ int2 mt_sh;
   const SweepView& V0 = views[0];
   int phase = 0;
@@ -1356,7 +1166,7 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
                                     &mt_sh, spin_limit(V0));
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
-    bwd_task(V, mt.y, *V.Lbase, 1, err, D, rinv, seg, zs);
+    bwd_task(V, mt.y, *V.Lbase, err, M);
   }
 }
 
@@ -2397,6 +2207,13 @@ static int persistent_grid(K kernel, size_t smem) {
   return std::max(1, sms) * std::max(1, per);
 }
 
+// The same for a kernel of single-column tasks (TaskSmem of shared memory).
+template <typename K>
+static int task_grid(K kernel) {
+  TEMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TaskSmem)));
+  return persistent_grid(kernel, sizeof(TaskSmem));
+}
+
 static void queued_views(temf_ctx& c, bool block, double* const* Lbase, double* x, SweepView& vf, SweepView& vb);
 static void reset_queues(temf_ctx& c, bool block, cudaStream_t st);
 
@@ -2589,13 +2406,8 @@ void launch_solve(temf_ctx& c, double* const* Lbase, double* x, int nrhs, cudaSt
     TEMF_CHECK_LAUNCH();
   }
   if (T.n_ftask) {
-    if (T.leaders) {
-      const int grid = std::min(persistent_grid(k_fwd_queued<true>, 0), T.n_ftask);
-      k_fwd_queued<true><<<grid, kSolveThreads, 0, st>>>(vf, c.d_status.p + 1);
-    } else {
-      const int grid = std::min(persistent_grid(k_fwd_queued<false>, 0), T.n_ftask);
-      k_fwd_queued<false><<<grid, kSolveThreads, 0, st>>>(vf, c.d_status.p + 1);
-    }
+    const auto kernel = T.leaders ? k_fwd_queued<true> : k_fwd_queued<false>;
+    kernel<<<std::min(task_grid(kernel), T.n_ftask), kSolveThreads, sizeof(TaskSmem), st>>>(vf, c.d_status.p + 1);
     TEMF_CHECK_LAUNCH();
   }
   if (inject) {
@@ -2605,13 +2417,8 @@ void launch_solve(temf_ctx& c, double* const* Lbase, double* x, int nrhs, cudaSt
   if (sgn) scale_rows(c, sgn, x, 1, 1, st);  // indefinite factor: L S L^T
   TEMF_CUDA(cudaMemsetAsync(T.bacc.p, 0, (size_t)c.n_edges * sizeof(double), st));
   if (T.n_btask) {
-    if (T.leaders) {
-      const int gridb = std::min(persistent_grid(k_bwd_queued<true>, 0), T.n_btask);
-      k_bwd_queued<true><<<gridb, kSolveThreads, 0, st>>>(vb, c.d_status.p + 1);
-    } else {
-      const int gridb = std::min(persistent_grid(k_bwd_queued<false>, 0), T.n_btask);
-      k_bwd_queued<false><<<gridb, kSolveThreads, 0, st>>>(vb, c.d_status.p + 1);
-    }
+    const auto kernel = T.leaders ? k_bwd_queued<true> : k_bwd_queued<false>;
+    kernel<<<std::min(task_grid(kernel), T.n_btask), kSolveThreads, sizeof(TaskSmem), st>>>(vb, c.d_status.p + 1);
     TEMF_CHECK_LAUNCH();
   }
   if (T.ntree) {
@@ -2625,19 +2432,15 @@ void launch_solve(temf_ctx& c, double* const* Lbase, double* x, int nrhs, cudaSt
 
 void launch_solve_scratch(temf_ctx& c, double* const* Lbase, double* x, int* sync, double* part, int* err,
                           cudaStream_t st) {
-  FactorPlan& F = c.fplan;
   SolvePlan& P = c.splan;
-  const size_t smem = (size_t)(kSnCols + kChunkRows) * sizeof(double);
   TEMF_CUDA(cudaMemsetAsync(sync, 0, (4 * (size_t)P.nsn + 4) * sizeof(int), st));
-  const int grid = std::min(persistent_grid(k_fwd_persistent, smem), std::max(P.n_ftask, 1));
-  k_fwd_persistent<<<grid, kSolveThreads, smem, st>>>(P.n_ftask, P.ftask.p, F.sn_first.p, F.sn_rows_ptr.p,
-                                                      F.sn_rows.p, F.sn_Lptr.p, Lbase, x, 1, P.ftgt_ptr.p, P.ftgt.p,
-                                                      P.fexpect.p, sync, P.nsn, err);
+  const SweepView vf = fwd_view(c, Lbase, x, sync);
+  SweepView vb = bwd_view(c, Lbase, x, sync, part);
+  k_fwd_persistent<<<std::min(task_grid(k_fwd_persistent), std::max(P.n_ftask, 1)), kSolveThreads, sizeof(TaskSmem), st>>>(
+      vf, err);
   TEMF_CHECK_LAUNCH();
-  const int gridb = std::min(persistent_grid(k_bwd_persistent, smem), std::max(P.n_btask, 1));
-  k_bwd_persistent<<<gridb, kSolveThreads, smem, st>>>(P.n_btask, P.btask.p, F.sn_first.p, F.sn_rows_ptr.p,
-                                                       F.sn_rows.p, F.sn_Lptr.p, Lbase, x, 1, P.btgt_ptr.p, P.btgt.p,
-                                                       P.nchunk.p, P.part_off.p, part, sync, P.nsn, err);
+  k_bwd_persistent<<<std::min(task_grid(k_bwd_persistent), std::max(P.n_btask, 1)), kSolveThreads, sizeof(TaskSmem), st>>>(
+      vb, err);
   TEMF_CHECK_LAUNCH();
 }
 
@@ -2702,31 +2505,36 @@ SweepView fwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync) {
   SweepView v{P.ftask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.ftgt_ptr.p,
               P.ftgt.p, P.fexpect.p, nullptr, nullptr, nullptr, sync, P.nsn, P.n_ftask};
   v.spin = c.spin_limit;
+  v.Dptr = F.sn_Dptr.p;
   return v;
 }
 
-SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync) {
+SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync, double* part) {
   FactorPlan& F = c.fplan;
   SolvePlan& P = c.splan;
-  ensure_update_buffer(c, 1);
+  if (!part) {
+    ensure_update_buffer(c, 1);
+    part = c.d_part.p;
+  }
   SweepView v{P.btask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.btgt_ptr.p,
-              P.btgt.p, nullptr, P.nchunk.p, P.part_off.p, c.d_part.p, sync, P.nsn, P.n_btask};
+              P.btgt.p, nullptr, P.nchunk.p, P.part_off.p, part, sync, P.nsn, P.n_btask};
   v.spin = c.spin_limit;
+  v.Dptr = F.sn_Dptr.p;
   return v;
 }
 
 int models_grid(bool forward) {
-  return forward ? persistent_grid(k_fwd_models, 0) : persistent_grid(k_bwd_models, 0);
+  return forward ? task_grid(k_fwd_models) : task_grid(k_bwd_models);
 }
 
 void launch_solve_models(int nf, const int2* order_f, const SweepView* vf, int nb, const int2* order_b,
                          const SweepView* vb, const int* active, int* counters, int* err, int grid_f, int grid_b,
                          int qlim_f, int qlim_b, cudaStream_t st) {
-  k_fwd_models<<<std::max(1, std::min(grid_f, nf + qlim_f)), kSolveThreads, 0, st>>>(nf, order_f, vf, active,
-                                                                                      counters, err, qlim_f);
+  k_fwd_models<<<std::max(1, std::min(grid_f, nf + qlim_f)), kSolveThreads, sizeof(TaskSmem), st>>>(
+      nf, order_f, vf, active, counters, err, qlim_f);
   TEMF_CHECK_LAUNCH();
-  k_bwd_models<<<std::max(1, std::min(grid_b, nb + qlim_b)), kSolveThreads, 0, st>>>(nb, order_b, vb, active,
-                                                                                      counters + 1, err, qlim_b);
+  k_bwd_models<<<std::max(1, std::min(grid_b, nb + qlim_b)), kSolveThreads, sizeof(TaskSmem), st>>>(
+      nb, order_b, vb, active, counters + 1, err, qlim_b);
   TEMF_CHECK_LAUNCH();
 }
 

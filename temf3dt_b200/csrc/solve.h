@@ -39,8 +39,7 @@ struct SweepView {
   int spin = 0;            // iterations a device wait may spin before it gives up (0: the default)
   double* bacc = nullptr;  // backward, one column: chunk partial sums accumulated per column (FP64 atomics)
   // single column: offsets (from the panel base) of the factor's scaled copies
-  // of the diagonal blocks (unit lower triangle, reciprocal diagonal); null:
-  // the tasks read the blocks from the panels
+  // of the diagonal blocks (unit lower triangle, reciprocal diagonal)
   const int64_t* Dptr = nullptr;
 };
 
@@ -92,7 +91,7 @@ void launch_spmv(temf_ctx& c, const double* M, const double* x, double* y, int n
 // forward and one backward merged sweep over (model, task) lists.  counters:
 // two claim counters, cleared by the caller; err: timeout word.
 SweepView fwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync);
-SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync);
+SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync, double* part = nullptr);
 int models_grid(bool forward);
 // Autotuner of the sweeps' ready-queue split level (the supernodes below it
 // are scheduled through the queue, the ones above are claimed in order with
