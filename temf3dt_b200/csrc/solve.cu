@@ -157,12 +157,11 @@ __device__ __forceinline__ void subst_warp(const double* D, double* vs, int c) {
 
 // Lower triangle of a diagonal block's scaled copy Q (c x c, column-major)
 // into D (row-major) with asynchronous copies, issued before a dependency
-// wait.
-__device__ __forceinline__ void load_diag_scaled(double* D, const double* Q, int c) {
-  for (int idx = threadIdx.x; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx - j * c;
-    if (i >= j) cp_async8(&D[i * kLdD + j], Q + idx);
-  }
+// wait by the warps from `first` on, a column each.
+__device__ __forceinline__ void load_diag_scaled(double* D, const double* Q, int c, int first = 0) {
+  const int lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5) - first;
+  for (int j = (int)(threadIdx.x >> 5) - first; j < c; j += nw)
+    for (int i = j + lane; i < c; i += 32) cp_async8(&D[i * kLdD + j], Q + (int64_t)j * c + i);
 }
 // rows c .. up to the next multiple of eight: zero (the backward substitution reads them)
 __device__ __forceinline__ void zero_diag_tail(double* D, int c) {
@@ -405,7 +404,6 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
   if (T.kind == 0 && tid < 32) {
     // Warp 0 substitutes: its registers hold coefficients, so its share of
     // the first chunk waits in shared memory.
-    load_diag_scaled(M.D, Lb + V.Dptr[s], c);
     if (row_on)
       for (int j = 0; j < c; ++j) cp_async8(&M.rows[j][lane], Pc + (int64_t)j * ld + i);
     cp_async_wait_all();
@@ -435,7 +433,7 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
     FwdRegs R;
     pre_fwd(R, Pc, c, ld, i, row_on);
     if (T.kind == 0) {
-      load_diag_scaled(M.D, Lb + V.Dptr[s], c);
+      load_diag_scaled(M.D, Lb + V.Dptr[s], c, 1);
       cp_async_wait_all();
       __syncthreads();
     } else {
@@ -1185,7 +1183,7 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
 //    into one c x 64 block per supernode (zeroed before each sweep), so the
 //    diagonal task reads one block however many chunks the supernode has.
 // ---------------------------------------------------------------------------
-constexpr int kLdm = 72;  // padded leading dimension of the 64-wide shared tiles
+constexpr int kLdm = 68;  // leading dimension of the 64-wide shared tiles: DMMA fragments without bank conflicts
 
 __device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -1195,50 +1193,53 @@ __device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b
 
 
 struct MultiSmem {
-  double D[kSnCols][kSnCols + 1];
+  double D[kSnCols][kSnCols + 2];
   double rinv[kSnCols];
   double A[kSnCols * kLdm];  // panel block, [j][i] (column j of L21, rows of the chunk)
   double Y[kSnCols * kLdm];  // right-hand-side block, [row][col]
 };
 
-// C[m][n] += sum_k A(m,k) B(k,n) for a 64 x 64 tile; warps 2x2 of 32x32.
+// C[m][n] += sum_k A(m,k) B(k,n) for a 64 x 8 nt tile: warp w has rows 16 w ..
+// 16 w + 15, so that few columns shorten every warp's work.
 // A(m,k) = Am[m * sam + k * sak], B(k,n) = Bk[k * kLdm + n].
-__device__ __forceinline__ void mma_tile64(double acc[4][4][2], const double* Am, int sam, int sak,
-                                           const double* Bk, int kdim) {
+__device__ __forceinline__ void mma_tile64(double acc[2][8][2], const double* Am, int sam, int sak,
+                                           const double* Bk, int kdim, int nt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
   const int g = lane >> 2, q = lane & 3;
+#pragma unroll 2
   for (int k0 = 0; k0 < kdim; k0 += 4) {
-    double fa[4], fb[4];
+    double fa[2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) fa[a] = Am[(wr + a * 8 + g) * sam + (k0 + q) * sak];
+    for (int a = 0; a < 2; ++a) fa[a] = Am[(16 * warp + a * 8 + g) * sam + (k0 + q) * sak];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) fb[b] = Bk[(k0 + q) * kLdm + wc + b * 8 + g];
+    for (int b = 0; b < 8; ++b) {
+      if (b < nt) {  // uniform
+        const double fb = Bk[(k0 + q) * kLdm + b * 8 + g];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+        for (int a = 0; a < 2; ++a) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb);
+      }
+    }
   }
 }
 
 // store the accumulators of mma_tile64 to a [m][n] tile with leading dimension kLdm
-__device__ __forceinline__ void store_tile64(const double acc[4][4][2], double* C) {
+__device__ __forceinline__ void store_tile64(const double acc[2][8][2], double* C, int nt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
   const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) C[(wr + a * 8 + g) * kLdm + wc + b * 8 + 2 * q + e] = acc[a][b][e];
+    for (int b = 0; b < 8; ++b)
+      if (b < nt)
+        *reinterpret_cast<double2*>(C + (16 * warp + a * 8 + g) * kLdm + b * 8 + 2 * q) =
+            make_double2(acc[a][b][0], acc[a][b][1]);
 }
 
-__device__ __forceinline__ void zero_acc(double acc[4][4][2]) {
+__device__ __forceinline__ void zero_acc(double acc[2][8][2]) {
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < 8; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 }
 
 // panel rows [r0, r0+nr) x columns [0, c) of L21 into A[j][i] (zero padded to 64 x 64), asynchronously
@@ -1250,61 +1251,123 @@ __device__ __forceinline__ void load_panel_block_async(double* A, const double* 
     else A[j * kLdm + i] = 0.0;
   }
 }
-// lower triangle of the diagonal block into D[i][j], asynchronously (rinv after the wait)
-__device__ __forceinline__ void load_diag_async(double (*D)[kSnCols + 1], const double* P, int c, int64_t ld) {
-  for (int idx = threadIdx.x; idx < c * c; idx += blockDim.x) {
-    const int j = idx / c, i = idx % c;
-    if (i >= j) cp_async8(&D[i][j], P + (int64_t)j * ld + i);
-  }
+constexpr int kMultiPanel = 16;  // rows substituted at a time
+// lower triangle of the diagonal block into D[i][j], asynchronously (rinv
+// after the wait); zeros in the rows from c up to whole panels
+__device__ __forceinline__ void load_diag_async(MultiSmem& M, const double* P, int c, int64_t ld) {
+  for (int j = threadIdx.x >> 5; j < c; j += kSolveThreads / 32)
+    for (int i = j + (int)(threadIdx.x & 31); i < c; i += 32) cp_async8(&M.D[i][j], P + (int64_t)j * ld + i);
+  const int w = (c + kMultiPanel - 1) / kMultiPanel * kMultiPanel;
+  for (int idx = threadIdx.x; idx < (w - c) * kSnCols; idx += blockDim.x) M.D[c + idx / kSnCols][idx % kSnCols] = 0.0;
 }
 __device__ __forceinline__ void finish_diag(MultiSmem& M, int c) {
-  if ((int)threadIdx.x < c) M.rinv[threadIdx.x] = 1.0 / M.D[threadIdx.x][threadIdx.x];
+  if ((int)threadIdx.x < kSnCols) M.rinv[threadIdx.x] = (int)threadIdx.x < c ? 1.0 / M.D[threadIdx.x][threadIdx.x] : 0.0;
 }
 
-// Y[j][col] = x[rows[j]][col] for j < nr, col < k (zero elsewhere); every
-// load of a thread is issued before the first store.
-template <bool kContiguous>
-__device__ __forceinline__ void load_rows(double* Y, const double* x, int64_t ldx, int k, int nr, int f,
-                                          const int* __restrict__ rows) {
-  constexpr int kPer = kSnCols * kSnCols / kSolveThreads;
+// Y[j][col] = x[rows[j]][col] for j < nr, col < k, zero for the other j and
+// col below the power of two kp >= k; every load of a thread is issued before
+// the first store.
+template <bool kContiguous, int kLogKp>
+__device__ __forceinline__ void load_rows_kp(double* Y, const double* x, int64_t ldx, int k, int nr, int f,
+                                             const int* __restrict__ rows) {
+  constexpr int kPer = (kSnCols << kLogKp) / kSolveThreads;
   double v[kPer];
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int idx = threadIdx.x + u * kSolveThreads;
-    const int j = idx / kSnCols, col = idx % kSnCols;
+    const int j = idx >> kLogKp, col = idx & ((1 << kLogKp) - 1);
     const int64_t row = kContiguous ? (int64_t)(f + j) : (j < nr ? (int64_t)rows[j] : 0);
     v[u] = (j < nr && col < k) ? __ldcg(x + row * ldx + col) : 0.0;
   }
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int idx = threadIdx.x + u * kSolveThreads;
-    Y[(idx / kSnCols) * kLdm + idx % kSnCols] = v[u];
+    Y[(idx >> kLogKp) * kLdm + (idx & ((1 << kLogKp) - 1))] = v[u];
   }
 }
+// the power of two of columns that the threads are laid out over (8 to 64)
+__device__ __forceinline__ int multi_log_kp(int k) { return k > 32 ? 6 : (k > 16 ? 5 : (k > 8 ? 4 : 3)); }
+// x[f + j][col] = Y[j][col] for j < c, col < k
+__device__ __forceinline__ void store_rows(const double* Y, double* x, int64_t ldx, int k, int c, int f) {
+  const int log_kp = multi_log_kp(k), col = threadIdx.x & ((1 << log_kp) - 1);
+  for (int j = threadIdx.x >> log_kp; j < c; j += kSolveThreads >> log_kp)
+    if (col < k) x[(int64_t)(f + j) * ldx + col] = Y[j * kLdm + col];
+}
+template <bool kContiguous>
+__device__ __forceinline__ void load_rows(double* Y, const double* x, int64_t ldx, int k, int nr, int f,
+                                          const int* __restrict__ rows) {
+  if (k > 32) load_rows_kp<kContiguous, 6>(Y, x, ldx, k, nr, f, rows);
+  else if (k > 16) load_rows_kp<kContiguous, 5>(Y, x, ldx, k, nr, f, rows);
+  else if (k > 8) load_rows_kp<kContiguous, 4>(Y, x, ldx, k, nr, f, rows);
+  else load_rows_kp<kContiguous, 3>(Y, x, ldx, k, nr, f, rows);
+}
 
-// Y = L11^{-1} Y (forward) or L11^{-T} Y (backward) for 64 columns; two
-// threads per column (adjacent lanes) split the rows by parity.
-__device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, bool forward) {
-  const int col = threadIdx.x >> 1, h = threadIdx.x & 1;
+// Y = L11^{-1} Y (forward) or L11^{-T} Y (backward) for k columns, 16 rows at
+// a time: the products with the rows already solved are DMMA tiles that start
+// from the panel's entries, then one thread per column substitutes inside the
+// panel in registers.  Every entry gets its FMAs in the order of
+// column-by-column substitution (ascending going forward, descending going
+// backward: the fragments' four columns are taken in reverse there), so the
+// result does not depend on the panel width.  64 rows and columns: about 2 us;
+// column by column in shared memory it was 20, most of a level.
+template <bool kForward>
+__device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int np = (c + kMultiPanel - 1) / kMultiPanel;
   double* Y = M.Y;
-  if (forward) {
-    for (int j = 0; j < c; ++j) {
-      if ((j & 1) == h) Y[j * kLdm + col] *= M.rinv[j];
-      __syncwarp();
-      const double yj = Y[j * kLdm + col];
-      int i = j + 1;
-      if ((i & 1) != h) ++i;
-      for (; i < c; i += 2) Y[i * kLdm + col] -= M.D[i][j] * yj;
+  for (int pp = 0; pp < np; ++pp) {
+    const int p = kForward ? pp : np - 1 - pp, j0 = kMultiPanel * p;
+    if (pp > 0) {
+      for (int n0 = 16 * warp; n0 < k; n0 += 64) {  // 16 columns per warp
+        double acc[2][2][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const double2 v = *reinterpret_cast<const double2*>(Y + (j0 + 8 * a + g) * kLdm + n0 + 8 * b + 2 * q);
+            acc[a][b][0] = v.x;
+            acc[a][b][1] = v.y;
+          }
+        const int ks = kForward ? j0 / 4 : kMultiPanel * (np - 1 - p) / 4;  // steps of four solved rows
+#pragma unroll 4
+        for (int u = 0; u < ks; ++u) {
+          const int kk = kForward ? 4 * u + q : kMultiPanel * np - 1 - 4 * u - q;
+          double fa[2], fb[2];
+#pragma unroll
+          for (int a = 0; a < 2; ++a) fa[a] = kForward ? -M.D[j0 + 8 * a + g][kk] : -M.D[kk][j0 + 8 * a + g];
+#pragma unroll
+          for (int b = 0; b < 2; ++b) fb[b] = Y[kk * kLdm + n0 + 8 * b + g];
+#pragma unroll
+          for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            *reinterpret_cast<double2*>(Y + (j0 + 8 * a + g) * kLdm + n0 + 8 * b + 2 * q) =
+                make_double2(acc[a][b][0], acc[a][b][1]);
+      }
+      __syncthreads();
     }
-  } else {
-    for (int j = c - 1; j >= 0; --j) {
-      if ((j & 1) == h) Y[j * kLdm + col] *= M.rinv[j];
-      __syncwarp();
-      const double xj = Y[j * kLdm + col];
-      for (int i = h; i < j; i += 2) Y[i * kLdm + col] -= M.D[j][i] * xj;
+    if (tid < k) {
+      double y[kMultiPanel];
+#pragma unroll
+      for (int j = 0; j < kMultiPanel; ++j) y[j] = Y[(j0 + j) * kLdm + tid];
+#pragma unroll
+      for (int jj = 0; jj < kMultiPanel; ++jj) {
+        const int j = kForward ? jj : kMultiPanel - 1 - jj;
+        y[j] *= M.rinv[j0 + j];
+#pragma unroll
+        for (int i = 0; i < kMultiPanel; ++i)
+          if (kForward ? i > j : i < j) y[i] -= (kForward ? M.D[j0 + i][j0 + j] : M.D[j0 + j][j0 + i]) * y[j];
+      }
+#pragma unroll
+      for (int j = 0; j < kMultiPanel; ++j) Y[(j0 + j) * kLdm + tid] = y[j];
     }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, int ldx, int k, int* err) {
@@ -1316,6 +1379,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
   double* x = V.x;
   const int tid = threadIdx.x;
   const double* Lb = *V.Lbase;
+  const int nt = (k + 7) / 8, log_kp = multi_log_kp(k), col = tid & ((1 << log_kp) - 1);
   int phase = 0;
   for (;;) {
     const int t = next_task(V, V.sync + 4 * V.nsn, true, err, phase, &task_id);
@@ -1331,7 +1395,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
     const int nr = T.r1 - T.r0;
     // the factor does not depend on the sweep: start its copies before any wait
     if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async(M.D, P, c, ld);
+    if (T.kind == 0) load_diag_async(M, P, c, ld);
     if (tid == 0 && !in_queue(V, t)) {  // claimed in order: wait for the inputs
       if (T.kind == 0) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
       else wait_geq(ydone + s, 1, err, 2, spin_limit(V));
@@ -1343,11 +1407,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
     if (T.kind == 0) {
       finish_diag(M, c);
       __syncthreads();
-      diag_solve_block(M, c, true);
-      for (int idx = tid; idx < c * k; idx += blockDim.x) {
-        const int j = idx / k, col = idx % k;
-        x[(int64_t)(f + j) * ldx + col] = M.Y[j * kLdm + col];
-      }
+      diag_solve_block<true>(M, c, k);
+      store_rows(M.Y, x, ldx, k, c, f);
       __threadfence();
       __syncthreads();
       if (tid == 0) atomicExch(ydone + s, 1);
@@ -1357,17 +1418,14 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
     }
     if (nr > 0) {
       // U = L21[rows] Y_s (64 x 64 x c), then push -U into the rows' right-hand sides
-      double acc[4][4][2];
+      double acc[2][8][2];
       zero_acc(acc);
-      mma_tile64(acc, M.A, 1, kLdm, M.Y, (c + 3) & ~3);
+      mma_tile64(acc, M.A, 1, kLdm, M.Y, (c + 3) & ~3, nt);
       __syncthreads();
-      store_tile64(acc, M.A);  // reuse A as [row][col]
+      store_tile64(acc, M.A, nt);  // reuse A as [row][col]
       __syncthreads();
-      const int warp = tid >> 5, lane = tid & 31;
-      for (int i = warp; i < nr; i += kSolveThreads / 32) {
-        double* dst = x + (int64_t)V.sn_rows[rp + T.r0 + i] * ldx;
-        for (int col = lane; col < k; col += 32) atomicAdd(dst + col, -M.A[i * kLdm + col]);
-      }
+      for (int i = tid >> log_kp; i < nr; i += kSolveThreads >> log_kp)
+        if (col < k) atomicAdd(x + (int64_t)V.sn_rows[rp + T.r0 + i] * ldx + col, -M.A[i * kLdm + col]);
       __threadfence();
       __syncthreads();
       count_inputs(V, V.tgt_ptr[t], V.tgt_ptr[t + 1]);
@@ -1384,6 +1442,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
   double* x = V.x;
   const int tid = threadIdx.x;
   const double* Lb = *V.Lbase;
+  const int nt = (k + 7) / 8, log_kp = multi_log_kp(k), col = tid & ((1 << log_kp) - 1);
   int phase = 0;
   for (;;) {
     const int t = next_task(V, V.sync + 4 * V.nsn + 1, false, err, phase, &task_id);
@@ -1398,7 +1457,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
     const double* P = Lb + V.Lptr[s];
     const int nr = T.r1 - T.r0;
     if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async(M.D, P, c, ld);
+    if (T.kind == 0) load_diag_async(M, P, c, ld);
     if (!in_queue(V, t)) {  // claimed in order: wait for the inputs, one polling thread each
       const int q0 = V.tgt_ptr[t], nq = V.tgt_ptr[t + 1] - q0;
       for (int q = tid; q < nq; q += blockDim.x) wait_geq(xdone + V.tgt[q0 + q], 1, err, 3, spin_limit(V));
@@ -1409,19 +1468,18 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
     if (nr > 0) load_rows<false>(M.Y, x, ldx, k, nr, 0, V.sn_rows + rp + T.r0);
     cp_async_wait_all();
     __syncthreads();
-    double acc[4][4][2];
+    double acc[2][8][2];
     zero_acc(acc);
     if (nr > 0) {
-      mma_tile64(acc, M.A, kLdm, 1, M.Y, 64);
+      mma_tile64(acc, M.A, kLdm, 1, M.Y, (nr + 3) & ~3, nt);
       __syncthreads();
     }
     double* as = V.part + V.part_off[s] * kMultiCols;  // this supernode's c x 64 accumulator
     if (T.kind == 1) {
-      store_tile64(acc, M.Y);
+      store_tile64(acc, M.Y, nt);
       __syncthreads();
-      const int warp = tid >> 5, lane = tid & 31;
-      for (int j = warp; j < c; j += kSolveThreads / 32)
-        for (int col = lane; col < k; col += 32) atomicAdd(as + j * kMultiCols + col, M.Y[j * kLdm + col]);
+      for (int j = tid >> log_kp; j < c; j += kSolveThreads >> log_kp)
+        if (col < k) atomicAdd(as + j * kMultiCols + col, M.Y[j * kLdm + col]);
       __threadfence();
       __syncthreads();
       if (tid == 0) {
@@ -1432,11 +1490,10 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
     } else {
       // Z = Y_s - (first chunk, here) - (other chunks, accumulated); back-substitute
       finish_diag(M, c);
-      store_tile64(acc, M.A);  // first-chunk products as [j][col]
+      store_tile64(acc, M.A, nt);  // first-chunk products as [j][col]
       __syncthreads();
       const bool more = V.nchunk[s] > 1;
-      for (int idx = tid; idx < kSnCols * kSnCols; idx += blockDim.x) {
-        const int j = idx / kSnCols, col = idx % kSnCols;
+      for (int j = tid >> log_kp; j < kSnCols; j += kSolveThreads >> log_kp) {
         double v = 0.0;
         if (j < c && col < k) {
           v = __ldcg(x + (int64_t)(f + j) * ldx + col);
@@ -1446,11 +1503,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
         M.Y[j * kLdm + col] = v;
       }
       __syncthreads();
-      diag_solve_block(M, c, false);
-      for (int idx = tid; idx < c * k; idx += blockDim.x) {
-        const int j = idx / k, col = idx % k;
-        x[(int64_t)(f + j) * ldx + col] = M.Y[j * kLdm + col];
-      }
+      diag_solve_block<false>(M, c, k);
+      store_rows(M.Y, x, ldx, k, c, f);
       __threadfence();
       __syncthreads();
       if (tid == 0) atomicExch(xdone + s, 1);
