@@ -60,6 +60,7 @@ struct FactorPlan {
   // the same slot allocation: c x c column-major, row i scaled by 1/L_ii
   // (unit lower triangle below the diagonal) and 1/L_ii on the diagonal.
   DBuf<int64_t> sn_Dptr;       // per supernode: offset of its copy (from the panel base)
+  std::vector<int64_t> dptr;   // host copy
   int64_t dsc_len = 0;         // doubles of all copies
 };
 
@@ -71,6 +72,18 @@ struct SolveTask {
   int r0;
   int r1;
 };
+
+// What a single-column sweep task reads of the plan, in one 64-byte fetch (the
+// supernode's arrays are two dependent loads away from a SolveTask).
+struct alignas(16) TaskDesc {
+  int s, kind, r0, r1;         // as SolveTask
+  int f, c, ld, nchunk;        // first column, width, panel rows, row chunks of the supernode
+  int tgt0, ntgt;              // forward: its targets in the target list; backward: the owner it waits for, 0 or 1
+  int64_t panel;               // offset of row r0 of the rows below the block, from the panel base
+  int64_t diag;                // offset of the scaled copy of the block
+  int64_t rows;                // index of row r0 in the row lists
+};
+static_assert(sizeof(TaskDesc) == 64, "one task descriptor is four 16-byte loads");
 
 // Ready-queue scheduling of a pair of sweep schedules: diagonal task per
 // supernode (forward, backward), backward dependants and completion counts,
@@ -104,6 +117,7 @@ struct TreePlan {
   DBuf<SolveTask> ftask, btask;
   int n_ftask = 0, n_btask = 0;
   DBuf<int> ftgt_ptr, ftgt, fexpect, btgt_ptr, btgt;
+  DBuf<TaskDesc> fdesc, bdesc; // per claimable task
   QueuePlan q;
   DBuf<double> bacc;           // backward: per column, the sum of its supernode's chunk partials
   bool tuned = false;
@@ -121,6 +135,7 @@ struct SolvePlan {
   DBuf<int> nchunk;            // per supernode: row chunks of its panel
   DBuf<int64_t> part_off;      // per supernode: offset of its backward partial sums
   int64_t part_len = 0;
+  DBuf<TaskDesc> fdesc, bdesc; // per claimable task of the schedules above
   QueuePlan q1;                // ready-queue data of the schedules above
   // the same schedules with 64-row chunks for blocks of up to 64 right-hand sides
   DBuf<SolveTask> mftask, mbtask;

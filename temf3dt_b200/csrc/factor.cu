@@ -632,7 +632,8 @@ void build_factor_plan(temf_ctx& c) {
     }
     dp[S.nsn] = o;
     F.dsc_len = o - S.stored;
-    F.sn_Dptr.upload(dp.data(), dp.size(), st);
+    F.dptr = dp;
+    F.sn_Dptr.upload(F.dptr.data(), F.dptr.size(), st);
   }
   // position of global row i in the panel of supernode t (i >= first column of t)
   auto panel_row = [&](int t, int i) -> int64_t {

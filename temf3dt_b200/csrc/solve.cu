@@ -341,62 +341,80 @@ struct TaskSmem {
   double rows[kSnCols][32];  // forward diagonal task: the chunk rows of warp 0, which runs the substitution
   double ys[kSnCols];        // y_s going forward; z, then x_s going backward
   double seg[4][kSnCols];    // backward: per warp, the column sums over its rows
+  TaskDesc d[2];             // the running task and the one claimed for after it
+  int id[2];
+};
+
+// A task's claim ahead (in-order tasks): taken when the running task's inputs
+// are complete, so that no CTA sits on a task while it waits for another's
+// result, and read back after its publish: the claim's round trip overlaps the
+// task's own work.  No deadlock: the unfinished task with the smallest index
+// is running, or its holder runs a smaller one.  Warp 3 claims (warp 0
+// substitutes).
+struct ClaimAhead {
+  int* counter;  // null: no claim ahead
+  int lo, hi;
+  int id;
+  __device__ __forceinline__ void take() {
+    if (counter && threadIdx.x >= 96) {
+      id = 0;
+      if (threadIdx.x == 96) id = atomicAdd(counter, 1);
+    }
+  }
+  __device__ __forceinline__ void fetch(const SweepView& V, TaskSmem& M, int slot) {
+    if (counter && threadIdx.x >= 96) {
+      id = lo + __shfl_sync(0xffffffffu, id, 0);
+      if (id >= hi) id = -1;
+      const int k = threadIdx.x - 96;
+      if (id >= 0 && k < (int)(sizeof(TaskDesc) / 16))
+        reinterpret_cast<int4*>(&M.d[slot])[k] = __ldg(reinterpret_cast<const int4*>(V.desc + id) + k);
+      if (k == 0) M.id[slot] = id;
+    }
+  }
 };
 
 // The chunk's pushes and counts, after y_s is in ys: shared by both kinds of
 // forward task.
-__device__ __forceinline__ void fwd_publish(const SweepView& V, const SolveTask& T, int t, int64_t r, int tg_o, int tg_d,
-                                            int tg_ex) {
+__device__ __forceinline__ void fwd_publish(const SweepView& V, const TaskDesc& T, int t, int tg_o, int tg_d, int tg_ex,
+                                            ClaimAhead& next, TaskSmem& M, int slot) {
   int* ready = V.sync;
   const int tid = threadIdx.x;
   __threadfence();
   __syncthreads();
   if (T.kind == 0) {
     if (tid == 0) atomicExch(V.sync + V.nsn + T.s, 1);
-    if (V.queue) {  // y_s is out: the other row chunks of s are ready (they follow this task)
-      const int nx = max(1, (int)((r + kChunkRows - 1) / kChunkRows)) - 1;
-      for (int k = tid; k < nx; k += blockDim.x) q_push(V, t + 1 + k);
-    }
+    // y_s is out: the other row chunks of a queued task are ready (they follow it)
+    if (in_queue(V, t))
+      for (int k = tid; k < T.nchunk - 1; k += blockDim.x) q_push(V, t + 1 + k);
   }
-  if (T.r1 > T.r0) {
-    if (V.queue) {
-      if (tg_o >= 0) {
-        const int old = atomicAdd(ready + tg_o, 1);
-        if (in_queue(V, tg_d) && old == tg_ex - 1) q_push(V, tg_d);
-      }
-      count_inputs(V, V.tgt_ptr[t] + (int)blockDim.x, V.tgt_ptr[t + 1]);  // longer lists (none expected)
-    } else if (tid == 0) {
-      for (int q = V.tgt_ptr[t]; q < V.tgt_ptr[t + 1]; ++q) atomicAdd(ready + V.tgt[q], 1);
-    }
+  if (tg_o >= 0) {
+    const int old = atomicAdd(ready + tg_o, 1);
+    if (in_queue(V, tg_d) && old == tg_ex - 1) q_push(V, tg_d);
   }
+  next.fetch(V, M, slot ^ 1);
 }
 
-__device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M,
-                                         unsigned long long* stamp = nullptr) {
+// task t, its descriptor in M.d[slot]
+__device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M, int slot,
+                                         ClaimAhead& next, unsigned long long* stamp = nullptr) {
   int* ready = V.sync;
   int* ydone = V.sync + V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x, lane = tid & 31;
-  const SolveTask T = V.tasks[t];
-  const int s = T.s;
-  const int f = V.sn_first[s];
-  const int c = V.sn_first[s + 1] - f;
-  const int64_t rp = V.rows_ptr[s];
-  const int64_t r = V.rows_ptr[s + 1] - rp;
-  const int64_t ld = c + r;
-  const double* Pc = Lb + V.Lptr[s] + c;
-  const int i = T.r0 + tid;
-  const bool row_on = i < T.r1;
-  const int row_i = row_on ? V.sn_rows[rp + i] : 0;  // the row this thread pushes to (read before the wait)
+  const TaskDesc& T = M.d[slot];
+  const int s = T.s, f = T.f, c = T.c;
+  const int64_t ld = T.ld;
+  const double* Pc = Lb + T.panel;  // row r0 of the rows below the block
+  const bool row_on = T.r0 + tid < T.r1;
   const bool queued = in_queue(V, t);
-  // this thread's target supernode with its diagonal task and input count,
-  // read before the wait (a chunk of at most blockDim rows feeds at most
-  // blockDim supernodes: one entry per thread)
+  // the row this thread pushes to, and its target supernode with its diagonal
+  // task and input count (a chunk of at most blockDim rows feeds at most
+  // blockDim supernodes: one entry per thread), read before the wait
+  const int row_i = row_on ? V.sn_rows[T.rows + tid] : 0;
   int tg_o = -1, tg_d = -1, tg_ex = 0;
-  if (V.queue && T.r1 > T.r0) {
-    const int k = V.tgt_ptr[t] + tid;
-    if (k < V.tgt_ptr[t + 1]) {
-      tg_o = V.tgt[k];
+  if (tid < T.ntgt) {
+    tg_o = V.tgt[T.tgt0 + tid];
+    if (V.queue) {
       tg_d = V.diag_task[tg_o];
       tg_ex = V.expect[tg_o];
     }
@@ -405,7 +423,7 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
     // Warp 0 substitutes: its registers hold coefficients, so its share of
     // the first chunk waits in shared memory.
     if (row_on)
-      for (int j = 0; j < c; ++j) cp_async8(&M.rows[j][lane], Pc + (int64_t)j * ld + i);
+      for (int j = 0; j < c; ++j) cp_async8(&M.rows[j][lane], Pc + (int64_t)j * ld + tid);
     cp_async_wait_all();
     __syncthreads();
     if (lane == 0 && !queued) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
@@ -431,9 +449,9 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
     }
   } else {
     FwdRegs R;
-    pre_fwd(R, Pc, c, ld, i, row_on);
+    pre_fwd(R, Pc, c, ld, tid, row_on);
     if (T.kind == 0) {
-      load_diag_scaled(M.D, Lb + V.Dptr[s], c, 1);
+      load_diag_scaled(M.D, Lb + T.diag, c, 1);
       cp_async_wait_all();
       __syncthreads();
     } else {
@@ -443,24 +461,37 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
       if (tid < c) M.ys[tid] = __ldcg(x + f + tid);
     }
     __syncthreads();
+    next.take();
     if (row_on) atomicAdd(x + row_i, -fin_fwd(R, M.ys, c));
   }
-  fwd_publish(V, T, t, r, tg_o, tg_d, tg_ex);
+  fwd_publish(V, T, t, tg_o, tg_d, tg_ex, next, M, slot);
+}
+
+// This CTA's next in-order task without a claim ahead: claimed and its
+// descriptor read by every thread's warp 3, -1 when done.
+__device__ __forceinline__ void claim_now(const SweepView& V, TaskSmem& M, int slot, int* counter, int lo, int hi) {
+  ClaimAhead c{counter, lo, hi, 0};
+  c.take();
+  c.fetch(V, M, slot);
+  __syncthreads();
+}
+// descriptor of task t (handed out by the ready queue) into M.d[slot]
+__device__ __forceinline__ void load_desc(const SweepView& V, TaskSmem& M, int slot, int t) {
+  if (threadIdx.x < sizeof(TaskDesc) / 16)
+    reinterpret_cast<int4*>(&M.d[slot])[threadIdx.x] = __ldg(reinterpret_cast<const int4*>(V.desc + t) + threadIdx.x);
+  __syncthreads();
 }
 
 // All tasks claimed in schedule order (no queue): the allocation-free solve.
 __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_persistent(const SweepView V, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
-  __shared__ int task_id;
   const double* Lb = *V.Lbase;
-  for (;;) {
-    if (threadIdx.x == 0) task_id = atomicAdd(V.sync + 4 * V.nsn, 1);
-    __syncthreads();
-    const int t = task_id;
-    __syncthreads();
-    if (t >= V.ntask) break;
-    fwd_task(V, t, Lb, err, M);
+  ClaimAhead next{V.sync + 4 * V.nsn, 0, V.ntask, 0};
+  claim_now(V, M, 0, next.counter, next.lo, next.hi);
+  for (int slot = 0; M.id[slot] >= 0; slot ^= 1) {
+    fwd_task(V, M.id[slot], Lb, err, M, slot, next);
+    __syncthreads();  // the task claimed ahead
   }
 }
 
@@ -473,27 +504,22 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_persistent(const Sweep
 //     the owners of the first chunk's rows, z = y_s - partials (fixed order,
 //     so the backward sweep is deterministic), solve with L11^T, publish x_s.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M,
-                                         unsigned long long* stamp = nullptr) {
+__device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M, int slot,
+                                         ClaimAhead& next, unsigned long long* stamp = nullptr) {
   int* cdone = V.sync + 2 * V.nsn;
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x;
-  const SolveTask T = V.tasks[t];
-  const int s = T.s;
-  const int f = V.sn_first[s];
-  const int c = V.sn_first[s + 1] - f;
-  const int64_t rp = V.rows_ptr[s];
-  const int64_t r = V.rows_ptr[s + 1] - rp;
-  const int64_t ld = c + r;
-  const double* P = Lb + V.Lptr[s];
+  const TaskDesc& T = M.d[slot];
+  const int s = T.s, f = T.f, c = T.c;
+  const int64_t ld = T.ld;
   const int nr = T.r1 - T.r0;
   FwdRegs R;
-  if (nr > 0) pre_fwd(R, P + c, c, ld, T.r0 + tid, tid < nr);
+  pre_fwd(R, Lb + T.panel, c, ld, tid, tid < nr);  // always: R defined on every path keeps it out of the rest of the loop
   // one chunk row per thread: its index read before the wait
-  const int row_t = tid < nr ? V.sn_rows[rp + T.r0 + tid] : 0;
+  const int row_t = tid < nr ? V.sn_rows[T.rows + tid] : 0;
   if (T.kind == 0) {
-    load_diag_scaled(M.D, Lb + V.Dptr[s], c);
+    load_diag_scaled(M.D, Lb + T.diag, c);
     zero_diag_tail(M.D, c);
   }
   const bool queued = in_queue(V, t);
@@ -503,25 +529,25 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   // is still awaited (on the top chain that owner is the block just above,
   // finished last).
   const bool pre = T.kind == 0 && V.bacc != nullptr;
-  const bool more = V.nchunk[s] > 1;
+  const bool more = T.nchunk > 1;
   double y_pre = 0.0, acc_pre = 0.0;
   if (T.kind == 0 && tid < c) y_pre = __ldcg(x + f + tid);
   // the chunk's rows need their owners' x; the diagonal task also its other chunks
-  if (!queued) {  // one polling thread per owner (and one for the chunk count)
-    const int q0 = V.tgt_ptr[t], nq = V.tgt_ptr[t + 1] - q0;
+  if (!queued) {  // (one owner: build_sched)
     if (pre) {
-      if (tid == blockDim.x - 1) wait_geq(cdone + s, V.nchunk[s] - (nr > 0 ? 1 : 0), err, 4, spin_limit(V));
+      if (tid == blockDim.x - 1) wait_geq(cdone + s, T.nchunk - (nr > 0 ? 1 : 0), err, 4, spin_limit(V));
       __syncthreads();
       if (tid < c && more) acc_pre = __ldcg(V.bacc + f + tid);
     }
-    for (int q = tid; q < nq; q += blockDim.x) wait_geq(xdone + V.tgt[q0 + q], 1, err, 3, spin_limit(V));
+    if (tid == 0 && T.ntgt > 0) wait_geq(xdone + T.tgt0, 1, err, 3, spin_limit(V));
     if (!pre && T.kind == 0 && tid == blockDim.x - 1)
-      wait_geq(cdone + s, V.nchunk[s] - (nr > 0 ? 1 : 0), err, 4, spin_limit(V));
+      wait_geq(cdone + s, T.nchunk - (nr > 0 ? 1 : 0), err, 4, spin_limit(V));
   } else if (pre && tid < c && more) {
     acc_pre = __ldcg(V.bacc + f + tid);
   }
   __syncthreads();
   if (stamp && tid == 0) *stamp = gtime();
+  next.take();
   if (nr > 0) {  // nr <= blockDim.x: one row per thread
     bwd_row_sums(R, tid < nr ? __ldcg(x + row_t) : 0.0, M.seg);
     __syncthreads();
@@ -537,7 +563,7 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
     __syncthreads();
     if (tid == 0) {
       atomicAdd(cdone + s, 1);
-      if (V.queue) {
+      if (queued) {  // its diagonal task follows it in the queue range
         const int d = V.diag_task[s];
         if (in_queue(V, d) && atomicAdd(V.cnt + d, 1) == V.need[d] - 1) q_push(V, d);
       }
@@ -547,7 +573,7 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
     if (!pre && more) {
       // without accumulators: thread (j, h) sums the partials of chunks q = 1 + h, 3 + h, ...
       // with eight loads in flight; fixed order
-      const int nch = V.nchunk[s];
+      const int nch = T.nchunk;
       const double* pp = V.part + V.part_off[s];
       const int j = tid & (kSnCols - 1), h = tid / kSnCols;
       double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -586,20 +612,18 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
     if (tid == 0) atomicExch(xdone + s, 1);
     if (V.queue) count_owner_done(V, V.dep_ptr[s], V.dep_ptr[s + 1]);  // x_s is out: every queued task whose rows s owns
   }
+  next.fetch(V, M, slot ^ 1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_persistent(const SweepView V, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
-  __shared__ int task_id;
   const double* Lb = *V.Lbase;
-  for (;;) {
-    if (threadIdx.x == 0) task_id = atomicAdd(V.sync + 4 * V.nsn + 1, 1);
-    __syncthreads();
-    const int t = task_id;
-    __syncthreads();
-    if (t >= V.ntask) break;
-    bwd_task(V, t, Lb, err, M);
+  ClaimAhead next{V.sync + 4 * V.nsn + 1, 0, V.ntask, 0};
+  claim_now(V, M, 0, next.counter, next.lo, next.hi);
+  for (int slot = 0; M.id[slot] >= 0; slot ^= 1) {
+    bwd_task(V, M.id[slot], Lb, err, M, slot, next);
+    __syncthreads();  // the task claimed ahead
   }
 }
 
@@ -793,50 +817,67 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
 // Instantiated with and without run leaders: the leader code needs many more
 // registers, so the plans without leaders get three resident CTAs per SM
 // (168 registers) for both sweeps; the backward with leaders two.
-template <bool kLeaders>
-__global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView V, int* err) {
+template <bool kLeaders, bool kForward>
+__device__ __forceinline__ void queued_sweep(const SweepView& V, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   __shared__ double ring[kLeaders ? kRing : 1];
   __shared__ int task_id;
   const double* Lb = *V.Lbase;
-  int phase = 0;
-  for (;;) {
-    const int t = next_task(V, V.sync + 4 * V.nsn, true, err, phase, &task_id);
-    if (t < 0) break;
-    unsigned long long* rec = g_timeline_f ? g_timeline_f + 4 * (size_t)t : nullptr;
-    if (rec && threadIdx.x == 0) rec[0] = gtime();
-    if (kLeaders && (V.tasks[t].kind & 15) == 3) {
-      if (rec && threadIdx.x == 0) rec[1] = gtime();
-      fwd_leader(V, t, Lb, err, M, ring);
+  int* counter = V.sync + 4 * V.nsn + (kForward ? 0 : 1);
+  unsigned long long* tl = kForward ? g_timeline_f : g_timeline_b;
+  // two phases: the ready queue's range (the bottom of the tree: first going
+  // forward, last going backward) and the tasks claimed in schedule order,
+  // one ahead.  With run leaders none is claimed ahead: a leader waits for
+  // tasks claimed after it, which must not be held back behind another.
+  bool ahead = false;
+  for (int phase = 0, slot = 0;;) {
+    const bool queue = (phase == 0) == kForward;
+    int t = -1;
+    if (ahead) {
+      __syncthreads();
+      t = M.id[slot];
+    } else if (queue) {
+      if (V.queue) {
+        if (threadIdx.x == 0) task_id = q_pop(V.qhead, V.queue, V.q_hi - V.q_lo, err, spin_limit(V));
+        __syncthreads();
+        t = task_id;
+        if (t >= 0) load_desc(V, M, slot, t);
+      }
     } else {
-      fwd_task(V, t, Lb, err, M, rec ? rec + 1 : nullptr);
+      __syncthreads();  // the last task's descriptor has been read
+      claim_now(V, M, slot, counter, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo);
+      t = M.id[slot];
+    }
+    if (t < 0) {
+      ahead = false;
+      if (++phase == 2) break;
+      continue;
+    }
+    ClaimAhead next{!queue && !kLeaders ? counter : nullptr, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo, 0};
+    unsigned long long* rec = tl ? tl + 4 * (size_t)t : nullptr;
+    if (rec && threadIdx.x == 0) rec[0] = gtime();
+    if (kLeaders && (M.d[slot].kind & 15) == 3) {
+      if (rec && threadIdx.x == 0) rec[1] = gtime();
+      if (kForward) fwd_leader(V, t, Lb, err, M, ring);
+      else bwd_leader(V, t, Lb, err, M, ring);
+    } else if (kForward) {
+      fwd_task(V, t, Lb, err, M, slot, next, rec ? rec + 1 : nullptr);
+    } else {
+      bwd_task(V, t, Lb, err, M, slot, next, rec ? rec + 1 : nullptr);
     }
     if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
+    ahead = !queue && !kLeaders;
+    slot ^= ahead ? 1 : 0;
   }
 }
-
+template <bool kLeaders>
+__global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView V, int* err) {
+  queued_sweep<kLeaders, true>(V, err);
+}
 template <bool kLeaders>
 __global__ void __launch_bounds__(kSolveThreads, kLeaders ? 2 : 3) k_bwd_queued(const SweepView V, int* err) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
-  __shared__ double ring[kLeaders ? kRing : 1];
-  __shared__ int task_id;
-  const double* Lb = *V.Lbase;
-  int phase = 0;
-  for (;;) {
-    const int t = next_task(V, V.sync + 4 * V.nsn + 1, false, err, phase, &task_id);
-    if (t < 0) break;
-    unsigned long long* rec = g_timeline_b ? g_timeline_b + 4 * (size_t)t : nullptr;
-    if (rec && threadIdx.x == 0) rec[0] = gtime();
-    if (kLeaders && (V.tasks[t].kind & 15) == 3) {
-      if (rec && threadIdx.x == 0) rec[1] = gtime();
-      bwd_leader(V, t, Lb, err, M, ring);
-    } else {
-      bwd_task(V, t, Lb, err, M, rec ? rec + 1 : nullptr);
-    }
-    if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
-  }
+  queued_sweep<kLeaders, false>(V, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1146,7 +1187,9 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_models(int nstatic, co
                                     &mt_sh, spin_limit(V0));
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
-    fwd_task(V, mt.y, *V.Lbase, err, M);
+    ClaimAhead none{nullptr, 0, 0, 0};
+    load_desc(V, M, 0, mt.y);
+    fwd_task(V, mt.y, *V.Lbase, err, M, 0, none);
   }
 }
 
@@ -1164,7 +1207,9 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
                                     &mt_sh, spin_limit(V0));
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
-    bwd_task(V, mt.y, *V.Lbase, err, M);
+    ClaimAhead none{nullptr, 0, 0, 0};
+    load_desc(V, M, 0, mt.y);
+    bwd_task(V, mt.y, *V.Lbase, err, M, 0, none);
   }
 }
 
@@ -1816,6 +1861,42 @@ void build_sched(const Symbolic& S, int CH, Sched& o, int min_level = 0, int lea
     o.btp.push_back((int)o.btg.size());
   }
 }
+// Descriptors of the first n tasks of a schedule (see TaskDesc).
+std::vector<TaskDesc> task_descs(const Symbolic& S, const Sched& a, bool forward, const std::vector<int64_t>& dptr) {
+  const std::vector<SolveTask>& tasks = forward ? a.ft : a.bt;
+  const std::vector<int>&tp = forward ? a.ftp : a.btp, &tg = forward ? a.ftg : a.btg;
+  std::vector<TaskDesc> out(forward ? a.nf : a.nb);
+  for (size_t i = 0; i < out.size(); ++i) {
+    const SolveTask& T = tasks[i];
+    TaskDesc& d = out[i];
+    const int c = S.sn_first[T.s + 1] - S.sn_first[T.s];
+    const int r = (int)(S.sn_rows_ptr[T.s + 1] - S.sn_rows_ptr[T.s]);
+    d.s = T.s;
+    d.kind = T.kind;
+    d.r0 = T.r0;
+    d.r1 = T.r1;
+    d.f = S.sn_first[T.s];
+    d.c = c;
+    d.ld = c + r;
+    d.nchunk = a.nch[T.s];
+    d.ntgt = tp[i + 1] - tp[i];
+    d.tgt0 = forward ? tp[i] : (d.ntgt ? tg[tp[i]] : -1);
+    d.panel = S.sn_Lptr[T.s] + c + T.r0;
+    d.diag = dptr[T.s];
+    d.rows = S.sn_rows_ptr[T.s] + T.r0;
+    if (d.ntgt > (forward ? kSolveThreads : 1)) throw StateError("a sweep task with more targets than threads");
+  }
+  return out;
+}
+
+void upload_descs(const Symbolic& S, const Sched& a, const std::vector<int64_t>& dptr, DBuf<TaskDesc>& f,
+                  DBuf<TaskDesc>& b, cudaStream_t st) {
+  const std::vector<TaskDesc> hf = task_descs(S, a, true, dptr), hb = task_descs(S, a, false, dptr);
+  f.upload(hf.data(), hf.size(), st);
+  b.upload(hb.data(), hb.size(), st);
+  TEMF_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
+}
+
 // Ready-queue data of a schedule: diagonal task per supernode (forward,
 // backward), backward completion counts and dependants, initially ready
 // tasks of both sweeps.
@@ -2167,6 +2248,7 @@ void upload_tree_plan(temf_ctx& c, int level, int split, bool leaders) {
   T.fexpect.upload(a.expect.data(), a.expect.size(), st);
   T.btgt_ptr.upload(a.btp.data(), a.btp.size(), st);
   T.btgt.upload(a.btg.data(), std::max<size_t>(a.btg.size(), 1), st);
+  upload_descs(S, a, c.fplan.dptr, T.fdesc, T.bdesc, st);
   upload_queue_plan(a, S, split, T.q, st);  // synchronises: the host vectors go out of scope
 }
 
@@ -2209,6 +2291,7 @@ void build_solve_plan(temf_ctx& c) {
   P.nchunk.upload(a.nch.data(), a.nch.size(), st);
   P.part_len = a.poff[nsn];
   P.part_off.upload(a.poff.data(), a.poff.size(), st);
+  upload_descs(S, a, c.fplan.dptr, P.fdesc, P.bdesc, st);
   upload_queue_plan(a, S, default_split(S), P.q1, st);
   TEMF_CUDA(cudaStreamSynchronize(st));  // the host vectors of `a` go out of scope
   upload_multi_plan(c, default_split(S));
@@ -2359,6 +2442,8 @@ static void tree_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& 
                  Q.b_lo, nb, 0, c.spin_limit};
   vb.bacc = T.bacc.p;  // allocated with the plan
   vf.Dptr = vb.Dptr = F.sn_Dptr.p;
+  vf.desc = T.fdesc.p;
+  vb.desc = T.bdesc.p;
 }
 
 static void reset_tree_queues(temf_ctx& c, cudaStream_t st) {
@@ -2559,7 +2644,7 @@ SweepView fwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync) {
   SweepView v{P.ftask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.ftgt_ptr.p,
               P.ftgt.p, P.fexpect.p, nullptr, nullptr, nullptr, sync, P.nsn, P.n_ftask};
   v.spin = c.spin_limit;
-  v.Dptr = F.sn_Dptr.p;
+  v.desc = P.fdesc.p;
   return v;
 }
 
@@ -2573,7 +2658,7 @@ SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync, doub
   SweepView v{P.btask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.btgt_ptr.p,
               P.btgt.p, nullptr, P.nchunk.p, P.part_off.p, part, sync, P.nsn, P.n_btask};
   v.spin = c.spin_limit;
-  v.Dptr = F.sn_Dptr.p;
+  v.desc = P.bdesc.p;
   return v;
 }
 
