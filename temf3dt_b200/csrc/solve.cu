@@ -175,20 +175,37 @@ __device__ __forceinline__ void zero_diag_tail(double* D, int c) {
 struct FwdRegs {
   double v[kSnCols];
 };
-__device__ __forceinline__ void pre_fwd(FwdRegs& R, const double* Pc, int c, int64_t ld, int i, bool on) {
+// Row `i` of the chunk (nr rows from Pc on), eight columns at a time while
+// there are any; columns past c repeat the last one and rows past nr the last
+// row, which the consumers multiply by zero or do not write.
+__device__ __forceinline__ void pre_fwd(FwdRegs& R, const double* Pc, int c, int64_t ld, int i, int nr) {
+  const double* p = Pc + max(min(i, nr - 1), 0);
 #pragma unroll
-  for (int j = 0; j < kSnCols; ++j) R.v[j] = (on && j < c) ? __ldg(Pc + (int64_t)j * ld + i) : 0.0;
+  for (int g = 0; g < kSnCols; g += 8) {
+    if (g < c && nr > 0) {  // uniform
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        R.v[g + u] = __ldg(p);
+        p += g + u + 1 < c ? ld : 0;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) R.v[g + u] = 0.0;
+    }
+  }
 }
-__device__ __forceinline__ double fin_fwd(const FwdRegs& R, const double* ys, int c) {
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+// ys: zero from c on
+__device__ __forceinline__ double fin_fwd(const FwdRegs& R, const double* ys) {
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int j = 0; j < kSnCols; j += 4) {
-    a0 += R.v[j] * (j < c ? ys[j] : 0.0);
-    a1 += R.v[j + 1] * (j + 1 < c ? ys[j + 1] : 0.0);
-    a2 += R.v[j + 2] * (j + 2 < c ? ys[j + 2] : 0.0);
-    a3 += R.v[j + 3] * (j + 3 < c ? ys[j + 3] : 0.0);
+    const double2 y0 = *reinterpret_cast<const double2*>(ys + j), y1 = *reinterpret_cast<const double2*>(ys + j + 2);
+    a[0] += R.v[j] * y0.x;
+    a[1] += R.v[j + 1] * y0.y;
+    a[2] += R.v[j + 2] * y1.x;
+    a[3] += R.v[j + 3] * y1.y;
   }
-  return (a0 + a1) + (a2 + a3);
+  return (a[0] + a[1]) + (a[2] + a[3]);
 }
 
 // Sum over the 32 lanes of each of the 32 per-lane values a[0..31]: lane l
@@ -436,7 +453,9 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
     __syncwarp();
     subst_warp<true>(M.D, M.ys, c);
     if (lane < c) x[f + lane] = M.ys[lane];
+    else M.ys[lane] = 0.0;
     if (lane + 32 < c) x[f + 32 + lane] = M.ys[lane + 32];
+    else M.ys[lane + 32] = 0.0;
     // y_s is published together with the first chunk's pushes below: one fence for both
     __syncthreads();
     if (row_on) {
@@ -449,7 +468,7 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
     }
   } else {
     FwdRegs R;
-    pre_fwd(R, Pc, c, ld, tid, row_on);
+    pre_fwd(R, Pc, c, ld, tid, T.r1 - T.r0);
     if (T.kind == 0) {
       load_diag_scaled(M.D, Lb + T.diag, c, 1);
       cp_async_wait_all();
@@ -458,11 +477,11 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
       if (tid == 0 && !queued) wait_geq(ydone + s, 1, err, 2, spin_limit(V));
       __syncthreads();
       if (stamp && tid == 0) *stamp = gtime();
-      if (tid < c) M.ys[tid] = __ldcg(x + f + tid);
+      if (tid < kSnCols) M.ys[tid] = tid < c ? __ldcg(x + f + tid) : 0.0;
     }
     __syncthreads();
     next.take();
-    if (row_on) atomicAdd(x + row_i, -fin_fwd(R, M.ys, c));
+    if (row_on) atomicAdd(x + row_i, -fin_fwd(R, M.ys));
   }
   fwd_publish(V, T, t, tg_o, tg_d, tg_ex, next, M, slot);
 }
@@ -515,7 +534,7 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   const int64_t ld = T.ld;
   const int nr = T.r1 - T.r0;
   FwdRegs R;
-  pre_fwd(R, Lb + T.panel, c, ld, tid, tid < nr);  // always: R defined on every path keeps it out of the rest of the loop
+  pre_fwd(R, Lb + T.panel, c, ld, tid, nr);  // always: R defined on every path keeps it out of the rest of the loop
   // one chunk row per thread: its index read before the wait
   const int row_t = tid < nr ? V.sn_rows[T.rows + tid] : 0;
   if (T.kind == 0) {
@@ -667,7 +686,7 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
     const int c = V.sn_first[a + 1] - f_run;
     const int64_t r = V.rows_ptr[a + 1] - V.rows_ptr[a], ld = c + r;
     const double* P = Lb + V.Lptr[a];
-    pre_fwd(R, P + c, c, ld, tid, tid < (r < kChunkRows ? r : (int64_t)kChunkRows));
+    pre_fwd(R, P + c, c, ld, tid, (int)(r < kChunkRows ? r : (int64_t)kChunkRows));
     load_diag_scaled(M.D, Lb + V.Dptr[a], c);
   }
   for (int q = a; q <= e; ++q) {
@@ -688,11 +707,12 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
       for (int j = tid; j < kSnCols; j += 32) M.ys[j] = j < c ? M.ys[j] * M.D[j * kLdD + j] : 0.0;
       __syncwarp();
       subst_warp<true>(M.D, M.ys, c);
+      for (int j = c + tid; j < kSnCols; j += 32) M.ys[j] = 0.0;
     }
     __syncthreads();
     for (int j = tid; j < c; j += blockDim.x) x[f + j] = M.ys[j];
     if (tid < r1) {
-      const double v = fin_fwd(R, M.ys, c);
+      const double v = fin_fwd(R, M.ys);
       const int row = V.sn_rows[rp + tid];
       if (row < f_end) ring[(row - f_run) & (kRing - 1)] -= v;  // inside the run: one writer per row
       else atomicAdd(x + row, -v);
@@ -709,7 +729,7 @@ __device__ void fwd_leader(const SweepView& V, int t, const double* Lb, int* err
       const int fn = V.sn_first[q + 1], cn = V.sn_first[q + 2] - fn;
       const int64_t rn = V.rows_ptr[q + 2] - V.rows_ptr[q + 1], ldn = cn + rn;
       const double* Pn = Lb + V.Lptr[q + 1];
-      pre_fwd(R, Pn + cn, cn, ldn, tid, tid < (rn < kChunkRows ? rn : (int64_t)kChunkRows));
+      pre_fwd(R, Pn + cn, cn, ldn, tid, (int)(rn < kChunkRows ? rn : (int64_t)kChunkRows));
       load_diag_scaled(M.D, Lb + V.Dptr[q + 1], cn);
     }
   }
@@ -730,7 +750,7 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
     const int64_t r = V.rows_ptr[e + 1] - V.rows_ptr[e], ld = c + r;
     const double* P = Lb + V.Lptr[e];
     const int r1 = (int)(r < kChunkRows ? r : (int64_t)kChunkRows);
-    if (r1 > 0) pre_fwd(R, P + c, c, ld, tid, tid < r1);
+    pre_fwd(R, P + c, c, ld, tid, r1);
     load_diag_scaled(M.D, Lb + V.Dptr[e], c);
     zero_diag_tail(M.D, c);
   }
@@ -806,7 +826,7 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
       const int64_t rn = V.rows_ptr[q] - V.rows_ptr[q - 1], ldn = cn + rn;
       const double* Pn = Lb + V.Lptr[q - 1];
       const int r1n = (int)(rn < kChunkRows ? rn : (int64_t)kChunkRows);
-      if (r1n > 0) pre_fwd(R, Pn + cn, cn, ldn, tid, tid < r1n);
+      pre_fwd(R, Pn + cn, cn, ldn, tid, r1n);
       load_diag_scaled(M.D, Lb + V.Dptr[q - 1], cn);
       zero_diag_tail(M.D, cn);
     }
