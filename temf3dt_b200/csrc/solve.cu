@@ -93,7 +93,7 @@ __device__ __forceinline__ void wait_geq(const int* flag, int target, int* err, 
 // forward), the solution on return.  Rows from c up to the next multiple of
 // eight: any values going forward; going backward vs and the rows of D are
 // zero there.
-constexpr int kLdD = kSnCols + 1;  // rows and columns of the block without bank conflicts
+constexpr int kLdD = kSnCols + 2;  // 16-byte pairs along a row; rows and columns of the block without bank conflicts
 template <bool kForward>
 __device__ __forceinline__ void subst_warp(const double* D, double* vs, int c) {
   const int lane = threadIdx.x & 31;
@@ -104,7 +104,11 @@ __device__ __forceinline__ void subst_warp(const double* D, double* vs, int c) {
 #pragma unroll
     for (int i = 1; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < i; ++j) t[i * (i - 1) / 2 + j] = D[(k0 + i) * kLdD + k0 + j];
+      for (int j = 0; j < i; j += 2) {
+        const double2 p = *reinterpret_cast<const double2*>(D + (k0 + i) * kLdD + k0 + j);
+        t[i * (i - 1) / 2 + j] = p.x;
+        if (j + 1 < i) t[i * (i - 1) / 2 + j + 1] = p.y;
+      }
   };
   load_t(8 * (kForward ? 0 : nb - 1));
 #pragma unroll 1
@@ -118,9 +122,21 @@ __device__ __forceinline__ void subst_warp(const double* D, double* vs, int c) {
       y[j + 1] = p.y;
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      u0[j] = kForward ? D[lane * kLdD + k0 + j] : D[(k0 + j) * kLdD + lane];
-      u1[j] = kForward ? D[(lane + 32) * kLdD + k0 + j] : D[(k0 + j) * kLdD + lane + 32];
+    for (int j = 0; j < 8; j += 2) {
+      if (kForward) {
+        const double2 p = *reinterpret_cast<const double2*>(D + lane * kLdD + k0 + j);
+        const double2 q = *reinterpret_cast<const double2*>(D + (lane + 32) * kLdD + k0 + j);
+        u0[j] = p.x;
+        u0[j + 1] = p.y;
+        u1[j] = q.x;
+        u1[j + 1] = q.y;
+      } else {
+#pragma unroll
+        for (int e = j; e < j + 2; ++e) {
+          u0[e] = D[(k0 + e) * kLdD + lane];
+          u1[e] = D[(k0 + e) * kLdD + lane + 32];
+        }
+      }
     }
     if (kForward) {
 #pragma unroll
@@ -443,15 +459,23 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
       for (int j = 0; j < c; ++j) cp_async8(&M.rows[j][lane], Pc + (int64_t)j * ld + tid);
     cp_async_wait_all();
     __syncthreads();
-    if (lane == 0 && !queued) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
-    __syncwarp();
-    if (stamp && lane == 0) *stamp = gtime();
-    const double x0 = lane < c ? __ldcg(x + f + lane) : 0.0;
-    const double x1 = lane + 32 < c ? __ldcg(x + f + 32 + lane) : 0.0;
-    M.ys[lane] = lane < c ? x0 * M.D[lane * kLdD + lane] : 0.0;  // the copy's diagonal: 1 / L_ii
-    M.ys[lane + 32] = lane + 32 < c ? x1 * M.D[(lane + 32) * kLdD + lane + 32] : 0.0;
-    __syncwarp();
-    subst_warp<true>(M.D, M.ys, c);
+    // The first pass substitutes one block of whatever ys holds: it brings the
+    // code in before the wait (its first run took 5.6 thousand cycles on the
+    // top chain, the next 3.0).
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass == 1) {
+        if (lane == 0 && !queued) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
+        __syncwarp();
+        if (stamp && lane == 0) *stamp = gtime();
+        const double x0 = lane < c ? __ldcg(x + f + lane) : 0.0;
+        const double x1 = lane + 32 < c ? __ldcg(x + f + 32 + lane) : 0.0;
+        M.ys[lane] = lane < c ? x0 * M.D[lane * kLdD + lane] : 0.0;  // the copy's diagonal: 1 / L_ii
+        M.ys[lane + 32] = lane + 32 < c ? x1 * M.D[(lane + 32) * kLdD + lane + 32] : 0.0;
+        __syncwarp();
+      }
+      subst_warp<true>(M.D, M.ys, pass == 0 ? 1 : c);
+    }
     if (lane < c) x[f + lane] = M.ys[lane];
     else M.ys[lane] = 0.0;
     if (lane + 32 < c) x[f + 32 + lane] = M.ys[lane + 32];
