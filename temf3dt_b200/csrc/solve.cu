@@ -1282,53 +1282,50 @@ __device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b
 
 
 struct MultiSmem {
-  double D[kSnCols][kSnCols + 2];
+  double D[kSnCols][kSnCols + 2];  // the diagonal block: forward transposed, [column][row]; backward [row][column]
   double rinv[kSnCols];
   double A[kSnCols * kLdm];  // panel block, [j][i] (column j of L21, rows of the chunk)
   double Y[kSnCols * kLdm];  // right-hand-side block, [row][col]
+  int rows[kChunkRowsMulti]; // the chunk's rows
 };
 
-// C[m][n] += sum_k A(m,k) B(k,n) for a 64 x 8 nt tile: warp w has rows 16 w ..
+// C[m][n] += sum_k A(m,k) B(k,n) for a 64 x 8 NT tile: warp w has rows 16 w ..
 // 16 w + 15, so that few columns shorten every warp's work.
 // A(m,k) = Am[m * sam + k * sak], B(k,n) = Bk[k * kLdm + n].
-__device__ __forceinline__ void mma_tile64(double acc[2][8][2], const double* Am, int sam, int sak,
-                                           const double* Bk, int kdim, int nt) {
+template <int NT>
+__device__ __forceinline__ void mma_tile64(double (&acc)[2][NT][2], const double* Am, int sam, int sak,
+                                           const double* Bk, int kdim) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < NT; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
 #pragma unroll 2
   for (int k0 = 0; k0 < kdim; k0 += 4) {
-    double fa[2];
+    double fa[2], fb[NT];
 #pragma unroll
     for (int a = 0; a < 2; ++a) fa[a] = Am[(16 * warp + a * 8 + g) * sam + (k0 + q) * sak];
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      if (b < nt) {  // uniform
-        const double fb = Bk[(k0 + q) * kLdm + b * 8 + g];
+    for (int b = 0; b < NT; ++b) fb[b] = Bk[(k0 + q) * kLdm + b * 8 + g];
 #pragma unroll
-        for (int a = 0; a < 2; ++a) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb);
-      }
-    }
+    for (int b = 0; b < NT; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
   }
 }
 
 // store the accumulators of mma_tile64 to a [m][n] tile with leading dimension kLdm
-__device__ __forceinline__ void store_tile64(const double acc[2][8][2], double* C, int nt) {
+template <int NT>
+__device__ __forceinline__ void store_tile64(const double (&acc)[2][NT][2], double* C) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, q = lane & 3;
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 8; ++b)
-      if (b < nt)
-        *reinterpret_cast<double2*>(C + (16 * warp + a * 8 + g) * kLdm + b * 8 + 2 * q) =
-            make_double2(acc[a][b][0], acc[a][b][1]);
-}
-
-__device__ __forceinline__ void zero_acc(double acc[2][8][2]) {
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < NT; ++b)
+      *reinterpret_cast<double2*>(C + (16 * warp + a * 8 + g) * kLdm + b * 8 + 2 * q) =
+          make_double2(acc[a][b][0], acc[a][b][1]);
 }
 
 // panel rows [r0, r0+nr) x columns [0, c) of L21 into A[j][i] (zero padded to 64 x 64), asynchronously
@@ -1341,54 +1338,58 @@ __device__ __forceinline__ void load_panel_block_async(double* A, const double* 
   }
 }
 constexpr int kMultiPanel = 16;  // rows substituted at a time
-// lower triangle of the diagonal block into D[i][j], asynchronously (rinv
-// after the wait); zeros in the rows from c up to whole panels
+// Lower triangle of the diagonal block into D, asynchronously; zeros in the
+// rows from c up to whole panels.
+template <bool kForward>
 __device__ __forceinline__ void load_diag_async(MultiSmem& M, const double* P, int c, int64_t ld) {
   for (int j = threadIdx.x >> 5; j < c; j += kSolveThreads / 32)
-    for (int i = j + (int)(threadIdx.x & 31); i < c; i += 32) cp_async8(&M.D[i][j], P + (int64_t)j * ld + i);
+    for (int i = j + (int)(threadIdx.x & 31); i < c; i += 32)
+      cp_async8(kForward ? &M.D[j][i] : &M.D[i][j], P + (int64_t)j * ld + i);
   const int w = (c + kMultiPanel - 1) / kMultiPanel * kMultiPanel;
-  for (int idx = threadIdx.x; idx < (w - c) * kSnCols; idx += blockDim.x) M.D[c + idx / kSnCols][idx % kSnCols] = 0.0;
+  for (int idx = threadIdx.x; idx < (w - c) * kSnCols; idx += blockDim.x) {
+    const int i = c + idx / kSnCols, j = idx % kSnCols;
+    if (kForward) M.D[j][i] = 0.0;
+    else M.D[i][j] = 0.0;
+  }
 }
 __device__ __forceinline__ void finish_diag(MultiSmem& M, int c) {
   if ((int)threadIdx.x < kSnCols) M.rinv[threadIdx.x] = (int)threadIdx.x < c ? 1.0 / M.D[threadIdx.x][threadIdx.x] : 0.0;
 }
 
-// Y[j][col] = x[rows[j]][col] for j < nr, col < k, zero for the other j and
-// col below the power of two kp >= k; every load of a thread is issued before
-// the first store.
-template <bool kContiguous, int kLogKp>
-__device__ __forceinline__ void load_rows_kp(double* Y, const double* x, int64_t ldx, int k, int nr, int f,
-                                             const int* __restrict__ rows) {
-  constexpr int kPer = (kSnCols << kLogKp) / kSolveThreads;
-  double v[kPer];
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int idx = threadIdx.x + u * kSolveThreads;
-    const int j = idx >> kLogKp, col = idx & ((1 << kLogKp) - 1);
-    const int64_t row = kContiguous ? (int64_t)(f + j) : (j < nr ? (int64_t)rows[j] : 0);
-    v[u] = (j < nr && col < k) ? __ldcg(x + row * ldx + col) : 0.0;
-  }
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int idx = threadIdx.x + u * kSolveThreads;
-    Y[(idx >> kLogKp) * kLdm + (idx & ((1 << kLogKp) - 1))] = v[u];
-  }
-}
-// the power of two of columns that the threads are laid out over (8 to 64)
-__device__ __forceinline__ int multi_log_kp(int k) { return k > 32 ? 6 : (k > 16 ? 5 : (k > 8 ? 4 : 3)); }
-// x[f + j][col] = Y[j][col] for j < c, col < k
-__device__ __forceinline__ void store_rows(const double* Y, double* x, int64_t ldx, int k, int c, int f) {
-  const int log_kp = multi_log_kp(k), col = threadIdx.x & ((1 << log_kp) - 1);
-  for (int j = threadIdx.x >> log_kp; j < c; j += kSolveThreads >> log_kp)
-    if (col < k) x[(int64_t)(f + j) * ldx + col] = Y[j * kLdm + col];
-}
-template <bool kContiguous>
+// The threads of a block-sweep task are laid out over 8 NT columns (16, 32 or
+// 64: the least that hold the k in use), element u of a thread being row
+// row(u), column col.
+template <int NT>
+struct MultiLayout {
+  static constexpr int kCols = 8 * NT, kPer = kSnCols * kCols / kSolveThreads;
+  static __device__ __forceinline__ int col() { return threadIdx.x % kCols; }
+  static __device__ __forceinline__ int row(int u) { return threadIdx.x / kCols + u * (kSolveThreads / kCols); }
+};
+// Y[j][col] = x[row j][col] for j < nr, col < k, zero elsewhere (row j: f + j,
+// or rows[j] when rows != null); every load of a thread is issued before the
+// first store.
+template <int NT>
 __device__ __forceinline__ void load_rows(double* Y, const double* x, int64_t ldx, int k, int nr, int f,
-                                          const int* __restrict__ rows) {
-  if (k > 32) load_rows_kp<kContiguous, 6>(Y, x, ldx, k, nr, f, rows);
-  else if (k > 16) load_rows_kp<kContiguous, 5>(Y, x, ldx, k, nr, f, rows);
-  else if (k > 8) load_rows_kp<kContiguous, 4>(Y, x, ldx, k, nr, f, rows);
-  else load_rows_kp<kContiguous, 3>(Y, x, ldx, k, nr, f, rows);
+                                          const int* rows) {
+  using G = MultiLayout<NT>;
+  double v[G::kPer];
+#pragma unroll
+  for (int u = 0; u < G::kPer; ++u) {
+    const int j = G::row(u);
+    v[u] = j < nr && G::col() < k ? __ldcg(x + (int64_t)(rows ? rows[j] : f + j) * ldx + G::col()) : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < G::kPer; ++u) Y[G::row(u) * kLdm + G::col()] = v[u];
+}
+// x[f + j][col] = Y[j][col] for j < c, col < k
+template <int NT>
+__device__ __forceinline__ void store_rows(const double* Y, double* x, int64_t ldx, int k, int c, int f) {
+  using G = MultiLayout<NT>;
+#pragma unroll 8
+  for (int u = 0; u < G::kPer; ++u) {
+    const int j = G::row(u);
+    if (j < c && G::col() < k) x[(int64_t)(f + j) * ldx + G::col()] = Y[j * kLdm + G::col()];
+  }
 }
 
 // Y = L11^{-1} Y (forward) or L11^{-T} Y (backward) for k columns, 16 rows at
@@ -1423,7 +1424,7 @@ __device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
           const int kk = kForward ? 4 * u + q : kMultiPanel * np - 1 - 4 * u - q;
           double fa[2], fb[2];
 #pragma unroll
-          for (int a = 0; a < 2; ++a) fa[a] = kForward ? -M.D[j0 + 8 * a + g][kk] : -M.D[kk][j0 + 8 * a + g];
+          for (int a = 0; a < 2; ++a) fa[a] = -M.D[kk][j0 + 8 * a + g];  // forward: the transposed block
 #pragma unroll
           for (int b = 0; b < 2; ++b) fb[b] = Y[kk * kLdm + n0 + 8 * b + g];
 #pragma unroll
@@ -1449,8 +1450,13 @@ __device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
         const int j = kForward ? jj : kMultiPanel - 1 - jj;
         y[j] *= M.rinv[j0 + j];
 #pragma unroll
-        for (int i = 0; i < kMultiPanel; ++i)
-          if (kForward ? i > j : i < j) y[i] -= (kForward ? M.D[j0 + i][j0 + j] : M.D[j0 + j][j0 + i]) * y[j];
+        for (int i = 0; i < kMultiPanel; i += 2) {  // the block's column (forward) or row j, in pairs
+          if (kForward ? i + 1 > j : i < j) {
+            const double2 p = *reinterpret_cast<const double2*>(&M.D[j0 + j][j0 + i]);
+            if (kForward ? i > j : i < j) y[i] -= p.x * y[j];
+            if (kForward ? i + 1 > j : i + 1 < j) y[i + 1] -= p.y * y[j];
+          }
+        }
       }
 #pragma unroll
       for (int j = 0; j < kMultiPanel; ++j) Y[(j0 + j) * kLdm + tid] = y[j];
@@ -1459,16 +1465,18 @@ __device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
   }
 }
 
+// NT: 8-column tiles the block is swept with (2, 4 or 8, the least that hold its columns).
+template <int NT>
 __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, int ldx, int k, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
   MultiSmem& M = *reinterpret_cast<MultiSmem*>(smraw);
+  using G = MultiLayout<NT>;
   __shared__ int task_id;
   int* ready = V.sync;
   int* ydone = V.sync + V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x;
   const double* Lb = *V.Lbase;
-  const int nt = (k + 7) / 8, log_kp = multi_log_kp(k), col = tid & ((1 << log_kp) - 1);
   int phase = 0;
   for (;;) {
     const int t = next_task(V, V.sync + 4 * V.nsn, true, err, phase, &task_id);
@@ -1482,56 +1490,71 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
     const int64_t ld = c + r;
     const double* P = Lb + V.Lptr[s];
     const int nr = T.r1 - T.r0;
-    // the factor does not depend on the sweep: start its copies before any wait
+    // what does not depend on the sweep comes before any wait: the factor's
+    // blocks, the rows, the targets (a chunk of 64 rows feeds at most 64
+    // supernodes: one per thread) and the reciprocal diagonal
     if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async(M, P, c, ld);
+    if (T.kind == 0) load_diag_async<true>(M, P, c, ld);
+    if (tid < nr) M.rows[tid] = V.sn_rows[rp + T.r0 + tid];
+    int tg_o = -1, tg_d = -1, tg_ex = 0;
+    if (nr > 0 && tid < V.tgt_ptr[t + 1] - V.tgt_ptr[t]) {
+      tg_o = V.tgt[V.tgt_ptr[t] + tid];
+      tg_d = V.diag_task[tg_o];
+      tg_ex = V.expect[tg_o];
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if (T.kind == 0) finish_diag(M, c);
     if (tid == 0 && !in_queue(V, t)) {  // claimed in order: wait for the inputs
       if (T.kind == 0) wait_geq(ready + s, V.expect[s], err, 1, spin_limit(V));
       else wait_geq(ydone + s, 1, err, 2, spin_limit(V));
     }
     __syncthreads();
-    load_rows<true>(M.Y, x, ldx, k, c, f, nullptr);
-    cp_async_wait_all();
+    load_rows<NT>(M.Y, x, ldx, k, c, f, nullptr);
     __syncthreads();
     if (T.kind == 0) {
-      finish_diag(M, c);
-      __syncthreads();
       diag_solve_block<true>(M, c, k);
-      store_rows(M.Y, x, ldx, k, c, f);
-      __threadfence();
+      store_rows<NT>(M.Y, x, ldx, k, c, f);  // published with the chunk's pushes below
+    }
+    if (nr > 0) {
+      // U = L21[rows] Y_s (64 x 8 NT x c), then push -U into the rows' right-hand sides
+      double acc[2][NT][2];
+      mma_tile64<NT>(acc, M.A, 1, kLdm, M.Y, (c + 3) & ~3);
       __syncthreads();
+      store_tile64<NT>(acc, M.A);  // reuse A as [row][col]
+      __syncthreads();
+#pragma unroll 8
+      for (int u = 0; u < G::kPer; ++u) {
+        const int i = G::row(u);
+        if (i < nr && G::col() < k) atomicAdd(x + (int64_t)M.rows[i] * ldx + G::col(), -M.A[i * kLdm + G::col()]);
+      }
+    }
+    __threadfence();
+    __syncthreads();
+    if (T.kind == 0) {
       if (tid == 0) atomicExch(ydone + s, 1);
       // y_s is out: the other row chunks of s (the tasks right after this one) are ready
       const int nx = max(1, (int)((r + kChunkRowsMulti - 1) / kChunkRowsMulti)) - 1;
       for (int q = tid; q < nx; q += blockDim.x) q_push(V, t + 1 + q);
     }
-    if (nr > 0) {
-      // U = L21[rows] Y_s (64 x 64 x c), then push -U into the rows' right-hand sides
-      double acc[2][8][2];
-      zero_acc(acc);
-      mma_tile64(acc, M.A, 1, kLdm, M.Y, (c + 3) & ~3, nt);
-      __syncthreads();
-      store_tile64(acc, M.A, nt);  // reuse A as [row][col]
-      __syncthreads();
-      for (int i = tid >> log_kp; i < nr; i += kSolveThreads >> log_kp)
-        if (col < k) atomicAdd(x + (int64_t)V.sn_rows[rp + T.r0 + i] * ldx + col, -M.A[i * kLdm + col]);
-      __threadfence();
-      __syncthreads();
-      count_inputs(V, V.tgt_ptr[t], V.tgt_ptr[t + 1]);
+    if (tg_o >= 0) {
+      const int old = atomicAdd(ready + tg_o, 1);
+      if (in_queue(V, tg_d) && old == tg_ex - 1) q_push(V, tg_d);
     }
   }
 }
 
+template <int NT>
 __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, int ldx, int k, int* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
   MultiSmem& M = *reinterpret_cast<MultiSmem*>(smraw);
+  using G = MultiLayout<NT>;
   __shared__ int task_id;
   int* cdone = V.sync + 2 * V.nsn;
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, col = G::col();
   const double* Lb = *V.Lbase;
-  const int nt = (k + 7) / 8, log_kp = multi_log_kp(k), col = tid & ((1 << log_kp) - 1);
   int phase = 0;
   for (;;) {
     const int t = next_task(V, V.sync + 4 * V.nsn + 1, false, err, phase, &task_id);
@@ -1546,7 +1569,11 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
     const double* P = Lb + V.Lptr[s];
     const int nr = T.r1 - T.r0;
     if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async(M, P, c, ld);
+    if (T.kind == 0) load_diag_async<false>(M, P, c, ld);
+    if (tid < nr) M.rows[tid] = V.sn_rows[rp + T.r0 + tid];
+    cp_async_wait_all();
+    __syncthreads();
+    if (T.kind == 0) finish_diag(M, c);
     if (!in_queue(V, t)) {  // claimed in order: wait for the inputs, one polling thread each
       const int q0 = V.tgt_ptr[t], nq = V.tgt_ptr[t + 1] - q0;
       for (int q = tid; q < nq; q += blockDim.x) wait_geq(xdone + V.tgt[q0 + q], 1, err, 3, spin_limit(V));
@@ -1554,21 +1581,20 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
     }
     __syncthreads();
     // Xr = x[rows] (64 x k); C = L21[rows]^T Xr (c x k)
-    if (nr > 0) load_rows<false>(M.Y, x, ldx, k, nr, 0, V.sn_rows + rp + T.r0);
-    cp_async_wait_all();
+    double acc[2][NT][2];
+    if (nr > 0) load_rows<NT>(M.Y, x, ldx, k, nr, 0, M.rows);
     __syncthreads();
-    double acc[2][8][2];
-    zero_acc(acc);
-    if (nr > 0) {
-      mma_tile64(acc, M.A, kLdm, 1, M.Y, (nr + 3) & ~3, nt);
-      __syncthreads();
-    }
+    mma_tile64<NT>(acc, M.A, kLdm, 1, M.Y, (nr + 3) & ~3);  // zeros without rows
+    __syncthreads();
     double* as = V.part + V.part_off[s] * kMultiCols;  // this supernode's c x 64 accumulator
     if (T.kind == 1) {
-      store_tile64(acc, M.Y, nt);
+      store_tile64<NT>(acc, M.Y);
       __syncthreads();
-      for (int j = tid >> log_kp; j < c; j += kSolveThreads >> log_kp)
-        if (col < k) atomicAdd(as + j * kMultiCols + col, M.Y[j * kLdm + col]);
+#pragma unroll 8
+      for (int u = 0; u < G::kPer; ++u) {
+        const int j = G::row(u);
+        if (j < c && col < k) atomicAdd(as + j * kMultiCols + col, M.Y[j * kLdm + col]);
+      }
       __threadfence();
       __syncthreads();
       if (tid == 0) {
@@ -1578,22 +1604,34 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
       }
     } else {
       // Z = Y_s - (first chunk, here) - (other chunks, accumulated); back-substitute
-      finish_diag(M, c);
-      store_tile64(acc, M.A, nt);  // first-chunk products as [j][col]
-      __syncthreads();
+      store_tile64<NT>(acc, M.A);  // first-chunk products as [j][col]
       const bool more = V.nchunk[s] > 1;
-      for (int j = tid >> log_kp; j < kSnCols; j += kSolveThreads >> log_kp) {
-        double v = 0.0;
-        if (j < c && col < k) {
-          v = __ldcg(x + (int64_t)(f + j) * ldx + col);
-          if (nr > 0) v -= M.A[j * kLdm + col];
-          if (more) v -= __ldcg(as + j * kMultiCols + col);
+      __syncthreads();
+      constexpr int kB = G::kPer < 16 ? G::kPer : 16;  // loads of a thread in flight
+#pragma unroll
+      for (int u0 = 0; u0 < G::kPer; u0 += kB) {
+        double v[kB], w[kB];
+#pragma unroll
+        for (int u = 0; u < kB; ++u) {
+          const int j = G::row(u0 + u);
+          const bool on = j < c && col < k;
+          v[u] = on ? __ldcg(x + (int64_t)(f + j) * ldx + col) : 0.0;
+          w[u] = on && more ? __ldcg(as + j * kMultiCols + col) : 0.0;
         }
-        M.Y[j * kLdm + col] = v;
+#pragma unroll
+        for (int u = 0; u < kB; ++u) {
+          const int j = G::row(u0 + u);
+          double z = v[u];
+          if (j < c && col < k) {
+            if (nr > 0) z -= M.A[j * kLdm + col];
+            if (more) z -= w[u];
+          }
+          M.Y[j * kLdm + col] = z;
+        }
       }
       __syncthreads();
       diag_solve_block<false>(M, c, k);
-      store_rows(M.Y, x, ldx, k, c, f);
+      store_rows<NT>(M.Y, x, ldx, k, c, f);
       __threadfence();
       __syncthreads();
       if (tid == 0) atomicExch(xdone + s, 1);
@@ -2404,20 +2442,22 @@ static void launch_solve_multi(temf_ctx& c, double* const* Lbase, double* x, int
                                const double* sgn) {
   SolvePlan& P = c.splan;
   const size_t smem = sizeof(MultiSmem);
-  TEMF_CUDA(cudaFuncSetAttribute(k_fwd_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  TEMF_CUDA(cudaFuncSetAttribute(k_bwd_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int gridf = std::min(persistent_grid(k_fwd_multi, smem), std::max(P.n_mftask, 1));
-  const int gridb = std::min(persistent_grid(k_bwd_multi, smem), std::max(P.n_mbtask, 1));
   for (int c0 = 0; c0 < nrhs; c0 += kMultiCols) {
     const int k = std::min(kMultiCols, nrhs - c0);
+    const auto fwd = k <= 16 ? k_fwd_multi<2> : (k <= 32 ? k_fwd_multi<4> : k_fwd_multi<8>);
+    const auto bwd = k <= 16 ? k_bwd_multi<2> : (k <= 32 ? k_bwd_multi<4> : k_bwd_multi<8>);
+    TEMF_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TEMF_CUDA(cudaFuncSetAttribute(bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int gridf = std::min(persistent_grid(fwd, smem), std::max(P.n_mftask, 1));
+    const int gridb = std::min(persistent_grid(bwd, smem), std::max(P.n_mbtask, 1));
     SweepView vf, vb;
     queued_views(c, true, Lbase, x + c0, vf, vb);
     reset_queues(c, true, st);
-    k_fwd_multi<<<gridf, kSolveThreads, smem, st>>>(vf, nrhs, k, c.d_status.p + 1);
+    fwd<<<gridf, kSolveThreads, smem, st>>>(vf, nrhs, k, c.d_status.p + 1);
     TEMF_CHECK_LAUNCH();
     if (sgn) scale_rows(c, sgn, x + c0, nrhs, k, st);  // indefinite factor: L S L^T
     TEMF_CUDA(cudaMemsetAsync(c.d_part.p, 0, (size_t)std::max<int64_t>(P.macc_len, 1) * kMultiCols * sizeof(double), st));
-    k_bwd_multi<<<gridb, kSolveThreads, smem, st>>>(vb, nrhs, k, c.d_status.p + 1);
+    bwd<<<gridb, kSolveThreads, smem, st>>>(vb, nrhs, k, c.d_status.p + 1);
     TEMF_CHECK_LAUNCH();
   }
 }
