@@ -119,7 +119,6 @@ struct TreePlan {
   DBuf<int> ftgt_ptr, ftgt, fexpect, btgt_ptr, btgt;
   DBuf<TaskDesc> fdesc, bdesc; // per claimable task
   QueuePlan q;
-  DBuf<double> bacc;           // backward: per column, the sum of its supernode's chunk partials
   bool tuned = false;
   std::vector<int> tune_level;  // per candidate (level, split) when tuned; splits and times in q
 };
@@ -145,8 +144,12 @@ struct SolvePlan {
   int64_t macc_len = 0;
   QueuePlan qm;
   TreePlan tree;               // the single-column sweeps of temf_solve / temf_run
-  DBuf<int> sync;              // ready | ydone | cdone | xdone (nsn each) | counters
+  // ready | ydone | cdone | xdone (nsn each) | counters | per column the sum of
+  // its supernode's backward chunk partials (single-column sweeps)
+  DBuf<int> sync;
   int nsn = 0;
+  size_t sync_words() const { return 4 * (size_t)nsn + 8; }  // even: the sums are 8-byte aligned
+  double* bacc() const { return reinterpret_cast<double*>(sync.p + sync_words()); }
 };
 
 struct FactorSlot {

@@ -2313,7 +2313,6 @@ void upload_tree_plan(temf_ctx& c, int level, int split, bool leaders) {
   build_sched(S, kChunkRows, a, level, leaders ? std::max(level, split) : INT_MAX, std::max(level, split));
   T.level = level;
   T.leaders = leaders;
-  if (T.bacc.n < (size_t)S.n) T.bacc.alloc(S.n);
   T.ntree = (int)trees.size();
   if (trees.empty()) T.trees.alloc(1);
   else T.trees.upload(trees.data(), trees.size(), st);
@@ -2335,9 +2334,12 @@ void upload_tree_plan(temf_ctx& c, int level, int split, bool leaders) {
 }
 
 // The highest subtree level (up to 11) below which there are still at least
-// min_roots subtrees.  The plan built with the analysis uses two subtrees per
-// resident warp of the subtree kernels (148 SMs x 12 warps).
-int default_tree_level(const Symbolic& S, int min_roots = 2 * 148 * 12) {
+// min_roots subtrees.  The plan built with the analysis asks for 2500, about
+// one and a half per resident warp of the subtree kernels: fewer leave warps
+// idle for the longest subtrees (301k edges: level 3 with 2666 subtrees 1.45 ms
+// a solve, level 4 with 1426 1.73, none 1.52; 1.48M: level 4 5.94, 5 6.10, 6
+// 6.70, none 6.53).
+int default_tree_level(const Symbolic& S, int min_roots = 2500) {
   int best = 0;
   for (int l = 1; l < std::min(S.nlevels, 12); ++l) {
     int roots = 0;
@@ -2377,8 +2379,14 @@ void build_solve_plan(temf_ctx& c) {
   upload_queue_plan(a, S, default_split(S), P.q1, st);
   TEMF_CUDA(cudaStreamSynchronize(st));  // the host vectors of `a` go out of scope
   upload_multi_plan(c, default_split(S));
-  P.sync.alloc(4 * (size_t)nsn + 8);  // + 2 claim counters of the task kernels, 2 of the subtree kernels
-  upload_tree_plan(c, default_tree_level(S), default_split(S), true);
+  // + 2 claim counters of the task kernels, 2 of the subtree kernels; then the backward column sums,
+  // cleared together
+  P.sync.alloc(P.sync_words() + 2 * (size_t)S.n);
+  // Until a tuned plan: every task claimed in order, one ahead, without run
+  // leaders (27k edges 0.27 ms a solve against 0.48 through the queue with
+  // leaders, 150k 0.86 against 2.0, 1.48M 6.1 against 11.5).
+  const int level = default_tree_level(S);
+  upload_tree_plan(c, level, level, false);
   P.tree.tuned = false;
   TEMF_CUDA(cudaStreamSynchronize(st));
 }
@@ -2497,7 +2505,7 @@ static void reset_queues(temf_ctx& c, bool block, cudaStream_t st) {
   const int nf = block ? P.n_mftask : P.n_ftask, nb = block ? P.n_mbtask : P.n_btask;
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;
-  TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync.bytes(), st));
+  TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync_words() * sizeof(int), st));
   TEMF_CUDA(cudaMemsetAsync(q, 0, Q.qbuf.bytes(), st));
   if (Q.n_finit)
     TEMF_CUDA(cudaMemcpyAsync(q, Q.finit.p, Q.n_finit * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -2505,6 +2513,10 @@ static void reset_queues(temf_ctx& c, bool block, cudaStream_t st) {
     TEMF_CUDA(cudaMemcpyAsync(q + nf, Q.binit.p, Q.n_binit * sizeof(int), cudaMemcpyDeviceToDevice, st));
   TEMF_CUDA(cudaMemcpyAsync(words + 2, Q.qtails.p, 2 * sizeof(int), cudaMemcpyDeviceToDevice, st));
 }
+
+// Whether the plan hands any task out through the ready queue (a queue split
+// at the subtree level leaves none: no queue to clear, seed or look up).
+static bool uses_queue(const TreePlan& T) { return T.q.f_hi > 0 || T.q.b_lo < T.n_btask; }
 
 // Views of the single-column sweeps of the tree plan: its task schedules
 // (the supernodes at or above the subtree level) with their ready queue.
@@ -2524,7 +2536,8 @@ static void tree_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& 
                  T.btgt.p, nullptr, P.nchunk.p, P.part_off.p, c.d_part.p, P.sync.p, P.nsn, nb,
                  q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
                  Q.b_lo, nb, 0, c.spin_limit};
-  vb.bacc = T.bacc.p;  // allocated with the plan
+  vb.bacc = P.bacc();
+  if (!uses_queue(T)) vf.queue = vb.queue = nullptr;
   vf.Dptr = vb.Dptr = F.sn_Dptr.p;
   vf.desc = T.fdesc.p;
   vb.desc = T.bdesc.p;
@@ -2537,7 +2550,8 @@ static void reset_tree_queues(temf_ctx& c, cudaStream_t st) {
   const int nf = T.n_ftask, nb = T.n_btask;
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;
-  TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync.bytes(), st));
+  TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync.bytes(), st));  // the sweep words and the column sums
+  if (!uses_queue(T)) return;
   TEMF_CUDA(cudaMemsetAsync(q, 0, Q.qbuf.bytes(), st));
   if (Q.n_finit)
     TEMF_CUDA(cudaMemcpyAsync(q, Q.finit.p, Q.n_finit * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -2638,7 +2652,6 @@ void launch_solve(temf_ctx& c, double* const* Lbase, double* x, int nrhs, cudaSt
     TEMF_CHECK_LAUNCH();
   }
   if (sgn) scale_rows(c, sgn, x, 1, 1, st);  // indefinite factor: L S L^T
-  TEMF_CUDA(cudaMemsetAsync(T.bacc.p, 0, (size_t)c.n_edges * sizeof(double), st));
   if (T.n_btask) {
     const auto kernel = T.leaders ? k_bwd_queued<true> : k_bwd_queued<false>;
     kernel<<<std::min(task_grid(kernel), T.n_btask), kSolveThreads, sizeof(TaskSmem), st>>>(vb, c.d_status.p + 1);
