@@ -47,11 +47,15 @@ struct FactorPlan {
   DBuf<int64_t> grp_relind;    // rel index of row 0 of the source (tables shared by the blocks of a run)
   DBuf<int> relind;
   DBuf<UpdTile> tiles;
-  std::vector<int64_t> tile_level_ptr;  // host, nlevels+1
+  // host, two parts per level: the tiles that the next level waits for, the others
+  struct UpdPart {
+    int64_t first = 0, count = 0;
+    int shape = 0;             // of the update kernel (factor.cu)
+  };
+  std::vector<UpdPart> upd;
   DBuf<int2> trsm;             // (supernode, first row) chunks of the row solves
   std::vector<int64_t> trsm_level_ptr;
   std::vector<int> level_width;  // host: widest supernode with rows below its block, per level
-  std::vector<int> upd_shape;    // host: shape of each level's update kernel (factor.cu)
   int64_t n_trsm = 0;
   int64_t n_relind = 0;
   int64_t n_tiles = 0;
@@ -150,6 +154,29 @@ struct SolvePlan {
   int nsn = 0;
   size_t sync_words() const { return 4 * (size_t)nsn + 8; }  // even: the sums are 8-byte aligned
   double* bacc() const { return reinterpret_cast<double*>(sync.p + sync_words()); }
+};
+
+// The factorisation's own stream (its chain of levels, at high priority) and
+// the events between it and the context's stream.
+struct FactorStreams {
+  cudaStream_t chain = nullptr;
+  cudaEvent_t chain_at = nullptr, rest_at = nullptr;
+  FactorStreams() = default;
+  FactorStreams(const FactorStreams&) = delete;
+  FactorStreams& operator=(const FactorStreams&) = delete;
+  void ensure() {
+    if (chain) return;
+    int least = 0, greatest = 0;
+    TEMF_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    TEMF_CUDA(cudaEventCreateWithFlags(&chain_at, cudaEventDisableTiming));
+    TEMF_CUDA(cudaEventCreateWithFlags(&rest_at, cudaEventDisableTiming));
+    TEMF_CUDA(cudaStreamCreateWithPriority(&chain, cudaStreamNonBlocking, greatest));
+  }
+  ~FactorStreams() {
+    if (chain_at) cudaEventDestroy(chain_at);
+    if (rest_at) cudaEventDestroy(rest_at);
+    if (chain) cudaStreamDestroy(chain);
+  }
 };
 
 struct FactorSlot {
@@ -258,6 +285,7 @@ struct temf_ctx {
   temf::FactorPlan fplan;
   temf::SolvePlan splan;
   temf::FactorSlot slots[2];
+  temf::FactorStreams fac;
   temf::DBuf<int> d_status;      // device status words (pivot failure etc.)
   temf::Source src;
   temf::Receivers rec;

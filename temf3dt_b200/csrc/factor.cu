@@ -700,7 +700,6 @@ void build_factor_plan(temf_ctx& c) {
     const std::vector<int> run_end = update_runs(S, kUpdMaxMembers);
     F.n_runs = 0;
     std::vector<UpdTile> tiles;
-    F.tile_level_ptr.assign(S.nlevels + 1, 0);
     // tiles of level l with edge T appended
     auto level_tiles = [&](int l, int T, std::vector<UpdTile>& out, bool count_runs) {
       for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
@@ -722,16 +721,40 @@ void build_factor_plan(temf_ctx& c) {
           for (int tj = 0; tj <= ti; ++tj) out.push_back({s, ti * T, tj * T, m});
       }
     };
-    F.upd_shape.assign(S.nlevels, kUpdWide);
-    for (int l = 0; l < S.nlevels; ++l) {
-      const size_t t0 = tiles.size();
-      level_tiles(l, kUpdTile, tiles, true);
-      F.upd_shape[l] = update_shape((int64_t)(tiles.size() - t0));
-      if (F.upd_shape[l] == kUpdSmall) {
-        tiles.resize(t0);
-        level_tiles(l, kUpdTile / 2, tiles, false);
+    // A level's tiles in two parts: those with a column of the next level's
+    // supernodes (the next level waits for them), then the others (by the 64
+    // columns a tile lies in, whatever its own size).
+    int flagged = -1;  // supernode of `flags`: per 64 columns, whether they hold one
+    std::vector<char> flags;
+    auto urgent = [&](const UpdTile& t, int l) {
+      if (t.s != flagged) {
+        flagged = t.s;
+        const int* rows = S.sn_rows.data() + S.sn_rows_ptr[t.s];
+        const int r = (int)nrows(t.s), jl = t.mj >> 4, n = jl > 0 ? std::min(jl, r) : r;
+        flags.assign(r / kUpdTile + 1, 0);
+        for (int j = 0; j < n; ++j)
+          if (S.sn_level[S.col2sn[rows[j]]] == l + 1) flags[j / kUpdTile] = 1;
       }
-      F.tile_level_ptr[l + 1] = (int64_t)tiles.size();
+      return flags[t.j0 / kUpdTile] != 0;
+    };
+    F.upd.assign(2 * (size_t)S.nlevels, FactorPlan::UpdPart{});
+    for (int l = 0; l < S.nlevels; ++l) {
+      std::vector<UpdTile> all, small, part[2];
+      level_tiles(l, kUpdTile, all, true);
+      for (const UpdTile& t : all) part[urgent(t, l) ? 0 : 1].push_back(t);
+      for (int k = 0; k < 2; ++k) {
+        FactorPlan::UpdPart& u = F.upd[2 * l + k];
+        u.shape = update_shape((int64_t)part[k].size());
+        if (u.shape == kUpdSmall && !part[k].empty()) {
+          if (small.empty()) level_tiles(l, kUpdTile / 2, small, false);
+          part[k].clear();
+          for (const UpdTile& t : small)
+            if (urgent(t, l) == (k == 0)) part[k].push_back(t);
+        }
+        u.first = (int64_t)tiles.size();
+        tiles.insert(tiles.end(), part[k].begin(), part[k].end());
+        u.count = (int64_t)tiles.size() - u.first;
+      }
     }
     F.n_tiles = (int64_t)tiles.size();
     F.tiles.upload(tiles.data(), tiles.size(), st);
@@ -818,33 +841,59 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   TEMF_CUDA(cudaFuncSetAttribute(upd_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<kUpdTile, 2>()));
   TEMF_CUDA(cudaFuncSetAttribute(upd_deep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<kUpdTile, 4>()));
   TEMF_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(kSnCols)));
+  const auto update = [&](const FactorPlan::UpdPart& u, cudaStream_t s) {
+    if (u.count == 0) return;
+    if (u.count > INT_MAX) throw StateError("too many update tiles in one level");
+    const auto upd = u.shape == kUpdWide ? upd_wide : (u.shape == kUpdDeep ? upd_deep : upd_small);
+    const size_t smem = u.shape == kUpdWide ? update_smem<kUpdTile, 2>()
+                                            : (u.shape == kUpdDeep ? update_smem<kUpdTile, 4>() : update_smem<kUpdTile / 2, 4>());
+    upd<<<(unsigned)u.count, 128, smem, s>>>(F.tiles.p + u.first, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p,
+                                             F.sn_Lptr.p, F.row_grp.p, F.grp_target.p, F.grp_shift.p, F.grp_relind.p,
+                                             F.relind.p, fs.L.p, sgn, c.d_status.p + 3);
+    TEMF_CHECK_LAUNCH();
+  };
+  // Two streams.  The chain (a level's blocks, its row solves, the updates
+  // the next level waits for) runs on a high-priority stream, the level's
+  // other updates on the context's stream, behind the next level's blocks and
+  // row solves (one CTA and a few, about 30 us).  A level's urgent updates
+  // wait for the other updates of the level before: every entry receives its
+  // levels' sums in the order of one stream.
+  FactorStreams& W = c.fac;
+  W.ensure();
+  const cudaStream_t hi = W.chain;
+  TEMF_CUDA(cudaEventRecord(W.chain_at, st));
+  TEMF_CUDA(cudaStreamWaitEvent(hi, W.chain_at, 0));
+  bool rest_pending = false;  // updates on st that the chain has not waited for
   for (int l = 0; l < S.nlevels; ++l) {
     const int cnt = S.level_ptr[l + 1] - S.level_ptr[l];
     if (cnt > 0) {
       const auto potrf = indefinite ? k_potrf<true> : k_potrf<false>;
-      potrf<<<cnt, kPotrfThreads, 0, st>>>(F.level_sn.p + S.level_ptr[l], F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p,
+      potrf<<<cnt, kPotrfThreads, 0, hi>>>(F.level_sn.p + S.level_ptr[l], F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p,
                                            fs.L.p, c.d_status.p, sgn, F.sn_Dptr.p);
       TEMF_CHECK_LAUNCH();
     }
     const int64_t c0 = F.trsm_level_ptr[l], c1 = F.trsm_level_ptr[l + 1];
     if (c1 > c0) {
-      k_trsm<<<(unsigned)(c1 - c0), kTrsmThreads, trsm_smem(F.level_width[l]), st>>>(
+      k_trsm<<<(unsigned)(c1 - c0), kTrsmThreads, trsm_smem(F.level_width[l]), hi>>>(
           reinterpret_cast<const TrsmChunk*>(F.trsm.p) + c0, F.sn_first.p, F.sn_rows_ptr.p, F.sn_Lptr.p, fs.L.p, sgn);
       TEMF_CHECK_LAUNCH();
     }
-    const int64_t t0 = F.tile_level_ptr[l], t1 = F.tile_level_ptr[l + 1];
-    if (t1 > t0) {
-      if (t1 - t0 > INT_MAX) throw StateError("too many update tiles in one level");
-      const int sh = F.upd_shape[l];
-      const auto upd = sh == kUpdWide ? upd_wide : (sh == kUpdDeep ? upd_deep : upd_small);
-      const size_t smem = sh == kUpdWide ? update_smem<kUpdTile, 2>()
-                                         : (sh == kUpdDeep ? update_smem<kUpdTile, 4>() : update_smem<kUpdTile / 2, 4>());
-      upd<<<(unsigned)(t1 - t0), 128, smem, st>>>(F.tiles.p + t0, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p,
-                                                  F.sn_Lptr.p, F.row_grp.p, F.grp_target.p, F.grp_shift.p,
-                                                  F.grp_relind.p, F.relind.p, fs.L.p, sgn, c.d_status.p + 3);
-      TEMF_CHECK_LAUNCH();
+    const FactorPlan::UpdPart &now = F.upd[2 * l], &rest = F.upd[2 * l + 1];
+    if (rest.count) TEMF_CUDA(cudaEventRecord(W.chain_at, hi));
+    if (rest_pending) {
+      TEMF_CUDA(cudaStreamWaitEvent(hi, W.rest_at, 0));
+      rest_pending = false;
+    }
+    update(now, hi);
+    if (rest.count) {
+      TEMF_CUDA(cudaStreamWaitEvent(st, W.chain_at, 0));
+      update(rest, st);
+      TEMF_CUDA(cudaEventRecord(W.rest_at, st));
+      rest_pending = true;
     }
   }
+  TEMF_CUDA(cudaEventRecord(W.chain_at, hi));
+  TEMF_CUDA(cudaStreamWaitEvent(st, W.chain_at, 0));
   fs.dt = b * 0.5;
   fs.valid = false;
 }
