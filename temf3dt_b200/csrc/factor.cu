@@ -409,14 +409,15 @@ __device__ __forceinline__ void mbar_wait(uint64_t* b, unsigned parity, int* err
 // the current chunk; the targets of the tile's columns are looked up
 // meanwhile.
 //
-// Tile size and buffers go by the tiles of the level (update_shape): a level
-// that gives every SM several 64 x 64 tiles is bound by the FP64 tensor pipe
-// and runs two buffers, five CTAs per SM; a smaller level is bound by the
-// latency of one tile, and four buffers hide the copies' (a 64 x 64 tile of
-// 512 columns on its own: 83 us with two buffers and a read-modify-write
-// scatter, 49 as 32 x 32 tiles); one that leaves SMs without a tile runs 32 x 32 tiles, four times
-// as many and a quarter as long.  An entry's sum runs over the same columns
-// in the same order in every shape.
+// Tile size and buffers go by the tiles launched together (update_shape).
+// More than one wave of 64 x 64 tiles with four buffers (three CTAs per SM):
+// two buffers and five CTAs per SM, bound by the FP64 tensor pipe (301k edges:
+// 18.3 ms a factorisation with the line at 3 tiles per SM, 18.8 at 8).  Up to
+// one wave is bound by the latency of a tile, and four buffers hide the
+// copies'.  Fewer tiles than SMs: 32 x 32 tiles, four times as many and a
+// quarter as long (a tile of 512 columns on its own: 83 us with two buffers
+// and a read-modify-write scatter, 49 as 32 x 32 tiles).  An entry's sum runs
+// over the same columns in the same order in every shape.
 constexpr int kUpdChunk = 16;
 constexpr int kUpdMaxMembers = 8;
 
@@ -581,11 +582,11 @@ __global__ void __launch_bounds__(128, kStages == 2 ? 5 : 3) k_update(
   }
 }
 
-// Shape of a level's update kernel by its number of 64 x 64 tiles.
+// Shape of an update launch by its number of 64 x 64 tiles.
 enum UpdShape { kUpdWide = 0, kUpdDeep = 1, kUpdSmall = 2 };
 constexpr int kSms = 148;
 inline UpdShape update_shape(int64_t tiles64) {
-  return tiles64 >= 8 * kSms ? kUpdWide : (tiles64 >= kSms ? kUpdDeep : kUpdSmall);
+  return tiles64 > 3 * kSms ? kUpdWide : (tiles64 >= kSms ? kUpdDeep : kUpdSmall);
 }
 
 // ---------------------------------------------------------------------------
