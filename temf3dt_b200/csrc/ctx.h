@@ -146,6 +146,7 @@ struct SolvePlan {
   DBuf<int> mftgt_ptr, mftgt, mfexpect, mbtgt_ptr, mbtgt, mnchunk;
   DBuf<int64_t> macc_off;      // per supernode with >= 2 chunks: row offset of its c x 64 accumulator
   int64_t macc_len = 0;
+  DBuf<TaskDesc> mfdesc, mbdesc;
   QueuePlan qm;
   TreePlan tree;               // the single-column sweeps of temf_solve / temf_run
   // ready | ydone | cdone | xdone (nsn each) | counters | per column the sum of

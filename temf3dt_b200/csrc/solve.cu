@@ -12,8 +12,8 @@
 //        every wait targets an earlier task, so no level barriers and no
 //        per-level launches; every wait is bounded and reports a timeout
 //        through an error word instead of hanging.  The forward sweep pushes
-//        row-chunk updates into the right-hand side with FP64 atomics; the
-//        backward sweep reduces in a fixed order.
+//        row-chunk updates into the right-hand side with FP64 atomics, the
+//        backward sweep adds its chunks' column sums the same way.
 //  * K6  ||a - b||^2 and ||b||^2 for the dt-doubling test (two_error,
 //        src/FETD_UTILITY.f90:578-599), fixed-order block reduction.
 //  * K7  receiver E and dB/dt from the six edge values of the receiver's
@@ -328,37 +328,6 @@ __device__ __forceinline__ int q_pop(int* qhead, const int* queue, int limit, in
   return v - 1;
 }
 
-// Next task of this CTA (every thread gets it; -1 when done).  Two phases:
-// the queue range through the ready queue, and the other tasks claimed in
-// schedule order from `counter` (with dependency waits).  Forward sweeps run
-// the queue phase first (their queue range is the bottom of the tree, at the
-// start of the schedule), backward sweeps last.  Without a queue every task
-// is claimed in order.
-__device__ __forceinline__ int next_task(const SweepView& V, int* counter, bool queue_first, int* err, int& phase,
-                                         int* sh) {
-  for (;;) {
-    const bool use_q = (phase == 0) == queue_first;
-    if (threadIdx.x == 0) {
-      int t = -1;
-      if (use_q) {
-        if (V.queue) t = q_pop(V.qhead, V.queue, V.q_hi - V.q_lo, err, spin_limit(V));
-      } else {
-        const bool front = V.queue == nullptr || V.q_lo > 0;  // static tasks before the queue range
-        const int lo = front ? 0 : V.q_hi, hi = V.queue == nullptr ? V.ntask : (front ? V.q_lo : V.ntask);
-        const int i = atomicAdd(counter, 1);
-        t = lo + i < hi ? lo + i : -1;
-      }
-      *sh = t;
-    }
-    __syncthreads();
-    const int t = *sh;
-    __syncthreads();
-    if (t >= 0) return t;
-    if (phase == 1) return -1;
-    phase = 1;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // forward  L y = b : persistent, dependency driven
 //   diagonal task of s (with its first row chunk): wait until every chunk that
@@ -368,14 +337,19 @@ __device__ __forceinline__ int next_task(const SweepView& V, int* counter, bool 
 //     ready counter of each supernode owning one of the rows;
 //   chunk task (s, r0..r1), r0 >= 128: wait for y_s, push the same way.
 // ---------------------------------------------------------------------------
+// The running task and the one claimed for after it.
+struct ClaimSlots {
+  TaskDesc d[2];
+  int id[2];
+};
+
 // Shared memory of the single-column tasks.
-struct TaskSmem {
+struct alignas(16) TaskSmem {
   double D[kSnCols * kLdD];
   double rows[kSnCols][32];  // forward diagonal task: the chunk rows of warp 0, which runs the substitution
   double ys[kSnCols];        // y_s going forward; z, then x_s going backward
   double seg[4][kSnCols];    // backward: per warp, the column sums over its rows
-  TaskDesc d[2];             // the running task and the one claimed for after it
-  int id[2];
+  ClaimSlots next;
 };
 
 // A task's claim ahead (in-order tasks): taken when the running task's inputs
@@ -394,7 +368,7 @@ struct ClaimAhead {
       if (threadIdx.x == 96) id = atomicAdd(counter, 1);
     }
   }
-  __device__ __forceinline__ void fetch(const SweepView& V, TaskSmem& M, int slot) {
+  __device__ __forceinline__ void fetch(const SweepView& V, ClaimSlots& M, int slot) {
     if (counter && threadIdx.x >= 96) {
       id = lo + __shfl_sync(0xffffffffu, id, 0);
       if (id >= hi) id = -1;
@@ -424,7 +398,7 @@ __device__ __forceinline__ void fwd_publish(const SweepView& V, const TaskDesc& 
     const int old = atomicAdd(ready + tg_o, 1);
     if (in_queue(V, tg_d) && old == tg_ex - 1) q_push(V, tg_d);
   }
-  next.fetch(V, M, slot ^ 1);
+  next.fetch(V, M.next, slot ^ 1);
 }
 
 // task t, its descriptor in M.d[slot]
@@ -434,7 +408,7 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
   int* ydone = V.sync + V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x, lane = tid & 31;
-  const TaskDesc& T = M.d[slot];
+  const TaskDesc& T = M.next.d[slot];
   const int s = T.s, f = T.f, c = T.c;
   const int64_t ld = T.ld;
   const double* Pc = Lb + T.panel;  // row r0 of the rows below the block
@@ -512,14 +486,14 @@ __device__ __forceinline__ void fwd_task(const SweepView& V, int t, const double
 
 // This CTA's next in-order task without a claim ahead: claimed and its
 // descriptor read by every thread's warp 3, -1 when done.
-__device__ __forceinline__ void claim_now(const SweepView& V, TaskSmem& M, int slot, int* counter, int lo, int hi) {
+__device__ __forceinline__ void claim_now(const SweepView& V, ClaimSlots& M, int slot, int* counter, int lo, int hi) {
   ClaimAhead c{counter, lo, hi, 0};
   c.take();
   c.fetch(V, M, slot);
   __syncthreads();
 }
 // descriptor of task t (handed out by the ready queue) into M.d[slot]
-__device__ __forceinline__ void load_desc(const SweepView& V, TaskSmem& M, int slot, int t) {
+__device__ __forceinline__ void load_desc(const SweepView& V, ClaimSlots& M, int slot, int t) {
   if (threadIdx.x < sizeof(TaskDesc) / 16)
     reinterpret_cast<int4*>(&M.d[slot])[threadIdx.x] = __ldg(reinterpret_cast<const int4*>(V.desc + t) + threadIdx.x);
   __syncthreads();
@@ -531,21 +505,22 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_persistent(const Sweep
   TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   const double* Lb = *V.Lbase;
   ClaimAhead next{V.sync + 4 * V.nsn, 0, V.ntask, 0};
-  claim_now(V, M, 0, next.counter, next.lo, next.hi);
-  for (int slot = 0; M.id[slot] >= 0; slot ^= 1) {
-    fwd_task(V, M.id[slot], Lb, err, M, slot, next);
+  claim_now(V, M.next, 0, next.counter, next.lo, next.hi);
+  for (int slot = 0; M.next.id[slot] >= 0; slot ^= 1) {
+    fwd_task(V, M.next.id[slot], Lb, err, M, slot, next);
     __syncthreads();  // the task claimed ahead
   }
 }
 
 // ---------------------------------------------------------------------------
 // backward  L^T x = y : persistent, dependency driven, top-down
-//   chunk task (s, r0..r1), r0 >= 128: wait for the supernodes owning those
-//     rows, stage x[rows] in shared memory, write the chunk's partial sums
-//     p_j = sum_i L21[i][j] x[rows_i];
+//   chunk task (s, r0..r1), r0 >= 128: wait for the owner of its lowest row,
+//     add p_j = sum_i L21[i][j] x[rows_i] to the column sums of s (FP64
+//     atomics; without them, in the allocation-free solve and the model
+//     batches, store it as the chunk's partial);
 //   diagonal task of s (with its first chunk): wait for the other chunks and
-//     the owners of the first chunk's rows, z = y_s - partials (fixed order,
-//     so the backward sweep is deterministic), solve with L11^T, publish x_s.
+//     the owner of the first chunk's lowest row, z = y_s - sums, solve with
+//     L11^T, publish x_s.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double* Lb, int* err, TaskSmem& M, int slot,
                                          ClaimAhead& next, unsigned long long* stamp = nullptr) {
@@ -553,12 +528,15 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x;
-  const TaskDesc& T = M.d[slot];
+  const TaskDesc& T = M.next.d[slot];
   const int s = T.s, f = T.f, c = T.c;
   const int64_t ld = T.ld;
   const int nr = T.r1 - T.r0;
   FwdRegs R;
-  pre_fwd(R, Lb + T.panel, c, ld, tid, nr);  // always: R defined on every path keeps it out of the rest of the loop
+  // Without a condition: rows defined on one branch only stayed live round the
+  // task loop, through the substitution, and half of them spilled (1.48M edges:
+  // 5.2 ms a sweep against 3.5).
+  pre_fwd(R, Lb + T.panel, c, ld, tid, nr);
   // one chunk row per thread: its index read before the wait
   const int row_t = tid < nr ? V.sn_rows[T.rows + tid] : 0;
   if (T.kind == 0) {
@@ -655,7 +633,7 @@ __device__ __forceinline__ void bwd_task(const SweepView& V, int t, const double
     if (tid == 0) atomicExch(xdone + s, 1);
     if (V.queue) count_owner_done(V, V.dep_ptr[s], V.dep_ptr[s + 1]);  // x_s is out: every queued task whose rows s owns
   }
-  next.fetch(V, M, slot ^ 1);
+  next.fetch(V, M.next, slot ^ 1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_persistent(const SweepView V, int* err) {
@@ -663,9 +641,9 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_persistent(const Sweep
   TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
   const double* Lb = *V.Lbase;
   ClaimAhead next{V.sync + 4 * V.nsn + 1, 0, V.ntask, 0};
-  claim_now(V, M, 0, next.counter, next.lo, next.hi);
-  for (int slot = 0; M.id[slot] >= 0; slot ^= 1) {
-    bwd_task(V, M.id[slot], Lb, err, M, slot, next);
+  claim_now(V, M.next, 0, next.counter, next.lo, next.hi);
+  for (int slot = 0; M.next.id[slot] >= 0; slot ^= 1) {
+    bwd_task(V, M.next.id[slot], Lb, err, M, slot, next);
     __syncthreads();  // the task claimed ahead
   }
 }
@@ -857,51 +835,62 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
   }
 }
 
-// The same sweeps scheduled through the ready queue (single right-hand side).
-// Instantiated with and without run leaders: the leader code needs many more
-// registers, so the plans without leaders get three resident CTAs per SM
-// (168 registers) for both sweeps; the backward with leaders two.
-template <bool kLeaders, bool kForward>
-__device__ __forceinline__ void queued_sweep(const SweepView& V, int* err) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
-  __shared__ double ring[kLeaders ? kRing : 1];
+// Hand-out of the tasks of a sweep, one at a time to run(task, slot, next),
+// in two phases: the ready queue's range (the bottom of the tree: first going
+// forward, last going backward) and the tasks claimed in schedule order, one
+// ahead where kAhead.
+template <bool kForward, bool kAhead, typename F>
+__device__ __forceinline__ void sweep_tasks(const SweepView& V, ClaimSlots& S, int* err, F&& run) {
   __shared__ int task_id;
-  const double* Lb = *V.Lbase;
   int* counter = V.sync + 4 * V.nsn + (kForward ? 0 : 1);
-  unsigned long long* tl = kForward ? g_timeline_f : g_timeline_b;
-  // two phases: the ready queue's range (the bottom of the tree: first going
-  // forward, last going backward) and the tasks claimed in schedule order,
-  // one ahead.  With run leaders none is claimed ahead: a leader waits for
-  // tasks claimed after it, which must not be held back behind another.
   bool ahead = false;
   for (int phase = 0, slot = 0;;) {
     const bool queue = (phase == 0) == kForward;
     int t = -1;
     if (ahead) {
       __syncthreads();
-      t = M.id[slot];
+      t = S.id[slot];
     } else if (queue) {
       if (V.queue) {
         if (threadIdx.x == 0) task_id = q_pop(V.qhead, V.queue, V.q_hi - V.q_lo, err, spin_limit(V));
         __syncthreads();
         t = task_id;
-        if (t >= 0) load_desc(V, M, slot, t);
+        if (t >= 0) load_desc(V, S, slot, t);
       }
     } else {
       __syncthreads();  // the last task's descriptor has been read
-      claim_now(V, M, slot, counter, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo);
-      t = M.id[slot];
+      claim_now(V, S, slot, counter, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo);
+      t = S.id[slot];
     }
     if (t < 0) {
       ahead = false;
       if (++phase == 2) break;
       continue;
     }
-    ClaimAhead next{!queue && !kLeaders ? counter : nullptr, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo, 0};
+    ClaimAhead next{!queue && kAhead ? counter : nullptr, kForward ? V.q_hi : 0, kForward ? V.ntask : V.q_lo, 0};
+    run(t, slot, next);
+    ahead = !queue && kAhead;
+    slot ^= ahead ? 1 : 0;
+  }
+}
+
+// With run leaders no task is claimed ahead: a leader waits for tasks claimed
+// after it, which must not be held back behind another.  The leader code needs
+// many more registers: without it both sweeps keep three CTAs per SM (168
+// registers; with two, without a spill, the backward sweep of the 1.48M-edge
+// mesh took 9.0 ms against 7.2 at three with spills), the backward sweep with
+// leaders two.
+template <bool kLeaders, bool kForward>
+__device__ __forceinline__ void queued_sweep(const SweepView& V, int* err) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TaskSmem& M = *reinterpret_cast<TaskSmem*>(smraw);
+  __shared__ double ring[kLeaders ? kRing : 1];
+  const double* Lb = *V.Lbase;
+  unsigned long long* tl = kForward ? g_timeline_f : g_timeline_b;
+  sweep_tasks<kForward, !kLeaders>(V, M.next, err, [&](int t, int slot, ClaimAhead& next) {
     unsigned long long* rec = tl ? tl + 4 * (size_t)t : nullptr;
     if (rec && threadIdx.x == 0) rec[0] = gtime();
-    if (kLeaders && (M.d[slot].kind & 15) == 3) {
+    if (kLeaders && (M.next.d[slot].kind & 15) == 3) {
       if (rec && threadIdx.x == 0) rec[1] = gtime();
       if (kForward) fwd_leader(V, t, Lb, err, M, ring);
       else bwd_leader(V, t, Lb, err, M, ring);
@@ -911,9 +900,7 @@ __device__ __forceinline__ void queued_sweep(const SweepView& V, int* err) {
       bwd_task(V, t, Lb, err, M, slot, next, rec ? rec + 1 : nullptr);
     }
     if (rec && threadIdx.x == 0) { rec[2] = gtime(); rec[3] = smid(); }
-    ahead = !queue && !kLeaders;
-    slot ^= ahead ? 1 : 0;
-  }
+  });
 }
 template <bool kLeaders>
 __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_queued(const SweepView V, int* err) {
@@ -1181,7 +1168,7 @@ __global__ void __launch_bounds__(kTreeThreads, 3) k_bwd_subtrees(const TreeView
 // where one small model alone leaves most SMs waiting.
 // ---------------------------------------------------------------------------
 // Next (model, task) of a merged sweep for this CTA; (-1, -1) when done.
-// Phase order as next_task: forward queue first, backward queue last.
+// Phase order as sweep_tasks: forward queue first, backward queue last.
 __device__ __forceinline__ int2 next_model_task(int nstatic, const int2* __restrict__ order,
                                                 const int* __restrict__ active, int* counter, int* qhead,
                                                 const int* queue, int qlim, bool queue_first, int* err, int& phase,
@@ -1232,7 +1219,7 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_fwd_models(int nstatic, co
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
     ClaimAhead none{nullptr, 0, 0, 0};
-    load_desc(V, M, 0, mt.y);
+    load_desc(V, M.next, 0, mt.y);
     fwd_task(V, mt.y, *V.Lbase, err, M, 0, none);
   }
 }
@@ -1252,7 +1239,7 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
     if (mt.x < 0) break;
     const SweepView V = views[mt.x];
     ClaimAhead none{nullptr, 0, 0, 0};
-    load_desc(V, M, 0, mt.y);
+    load_desc(V, M.next, 0, mt.y);
     bwd_task(V, mt.y, *V.Lbase, err, M, 0, none);
   }
 }
@@ -1266,7 +1253,8 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
 //  * right-hand-side rows are read with all of a thread's loads in flight at
 //    once (register staging; L2-coherent loads, since other CTAs write them);
 //  * the 64 x 64 x c chunk products run on the FP64 tensor cores (DMMA);
-//  * the c x 64 diagonal solves use two threads per column;
+//  * the diagonal solves take 16 rows at a time: DMMA for the rows before, one
+//    thread per column inside (diag_solve_block);
 //  * forward chunk updates are pushed into the ancestors' rows with FP64
 //    atomics; backward chunk partial sums are accumulated with FP64 atomics
 //    into one c x 64 block per supernode (zeroed before each sweep), so the
@@ -1281,12 +1269,13 @@ __device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b
 }
 
 
-struct MultiSmem {
+struct alignas(16) MultiSmem {
   double D[kSnCols][kSnCols + 2];  // the diagonal block: forward transposed, [column][row]; backward [row][column]
   double rinv[kSnCols];
   double A[kSnCols * kLdm];  // panel block, [j][i] (column j of L21, rows of the chunk)
   double Y[kSnCols * kLdm];  // right-hand-side block, [row][col]
   int rows[kChunkRowsMulti]; // the chunk's rows
+  ClaimSlots next;
 };
 
 // C[m][n] += sum_k A(m,k) B(k,n) for a 64 x 8 NT tile: warp w has rows 16 w ..
@@ -1328,12 +1317,11 @@ __device__ __forceinline__ void store_tile64(const double (&acc)[2][NT][2], doub
           make_double2(acc[a][b][0], acc[a][b][1]);
 }
 
-// panel rows [r0, r0+nr) x columns [0, c) of L21 into A[j][i] (zero padded to 64 x 64), asynchronously
-__device__ __forceinline__ void load_panel_block_async(double* A, const double* P, int c, int64_t ld, int r0,
-                                                       int nr) {
+// nr panel rows from Pc on x columns [0, c) of L21 into A[j][i] (zero padded to 64 x 64), asynchronously
+__device__ __forceinline__ void load_panel_block_async(double* A, const double* Pc, int c, int64_t ld, int nr) {
   for (int idx = threadIdx.x; idx < kSnCols * kSnCols; idx += blockDim.x) {
     const int j = idx / kSnCols, i = idx % kSnCols;
-    if (j < c && i < nr) cp_async8(A + j * kLdm + i, P + (int64_t)j * ld + c + r0 + i);
+    if (j < c && i < nr) cp_async8(A + j * kLdm + i, Pc + (int64_t)j * ld + i);
     else A[j * kLdm + i] = 0.0;
   }
 }
@@ -1471,36 +1459,29 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
   extern __shared__ __align__(16) unsigned char smraw[];
   MultiSmem& M = *reinterpret_cast<MultiSmem*>(smraw);
   using G = MultiLayout<NT>;
-  __shared__ int task_id;
   int* ready = V.sync;
   int* ydone = V.sync + V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x;
   const double* Lb = *V.Lbase;
-  int phase = 0;
-  for (;;) {
-    const int t = next_task(V, V.sync + 4 * V.nsn, true, err, phase, &task_id);
-    if (t < 0) break;
-    const SolveTask T = V.tasks[t];
-    const int s = T.s;
-    const int f = V.sn_first[s];
-    const int c = V.sn_first[s + 1] - f;
-    const int64_t rp = V.rows_ptr[s];
-    const int64_t r = V.rows_ptr[s + 1] - rp;
-    const int64_t ld = c + r;
-    const double* P = Lb + V.Lptr[s];
+  sweep_tasks<true, true>(V, M.next, err, [&](int t, int slot, ClaimAhead& next) {
+    const TaskDesc& T = M.next.d[slot];
+    const int s = T.s, f = T.f, c = T.c;
+    const int64_t ld = T.ld;
     const int nr = T.r1 - T.r0;
     // what does not depend on the sweep comes before any wait: the factor's
     // blocks, the rows, the targets (a chunk of 64 rows feeds at most 64
     // supernodes: one per thread) and the reciprocal diagonal
-    if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async<true>(M, P, c, ld);
-    if (tid < nr) M.rows[tid] = V.sn_rows[rp + T.r0 + tid];
+    if (nr > 0) load_panel_block_async(M.A, Lb + T.panel, c, ld, nr);
+    if (T.kind == 0) load_diag_async<true>(M, Lb + T.diag, c, ld);
+    if (tid < nr) M.rows[tid] = V.sn_rows[T.rows + tid];
     int tg_o = -1, tg_d = -1, tg_ex = 0;
-    if (nr > 0 && tid < V.tgt_ptr[t + 1] - V.tgt_ptr[t]) {
-      tg_o = V.tgt[V.tgt_ptr[t] + tid];
-      tg_d = V.diag_task[tg_o];
-      tg_ex = V.expect[tg_o];
+    if (tid < T.ntgt) {
+      tg_o = V.tgt[T.tgt0 + tid];
+      if (V.queue) {
+        tg_d = V.diag_task[tg_o];
+        tg_ex = V.expect[tg_o];
+      }
     }
     cp_async_wait_all();
     __syncthreads();
@@ -1510,6 +1491,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
       else wait_geq(ydone + s, 1, err, 2, spin_limit(V));
     }
     __syncthreads();
+    next.take();
     load_rows<NT>(M.Y, x, ldx, k, c, f, nullptr);
     __syncthreads();
     if (T.kind == 0) {
@@ -1533,15 +1515,16 @@ __global__ void __launch_bounds__(kSolveThreads) k_fwd_multi(const SweepView V, 
     __syncthreads();
     if (T.kind == 0) {
       if (tid == 0) atomicExch(ydone + s, 1);
-      // y_s is out: the other row chunks of s (the tasks right after this one) are ready
-      const int nx = max(1, (int)((r + kChunkRowsMulti - 1) / kChunkRowsMulti)) - 1;
-      for (int q = tid; q < nx; q += blockDim.x) q_push(V, t + 1 + q);
+      // y_s is out: the other row chunks of a queued task (they follow it) are ready
+      if (in_queue(V, t))
+        for (int q = tid; q < T.nchunk - 1; q += blockDim.x) q_push(V, t + 1 + q);
     }
     if (tg_o >= 0) {
       const int old = atomicAdd(ready + tg_o, 1);
       if (in_queue(V, tg_d) && old == tg_ex - 1) q_push(V, tg_d);
     }
-  }
+    next.fetch(V, M.next, slot ^ 1);
+  });
 }
 
 template <int NT>
@@ -1549,37 +1532,28 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
   extern __shared__ __align__(16) unsigned char smraw[];
   MultiSmem& M = *reinterpret_cast<MultiSmem*>(smraw);
   using G = MultiLayout<NT>;
-  __shared__ int task_id;
   int* cdone = V.sync + 2 * V.nsn;
   int* xdone = V.sync + 3 * V.nsn;
   double* x = V.x;
   const int tid = threadIdx.x, col = G::col();
   const double* Lb = *V.Lbase;
-  int phase = 0;
-  for (;;) {
-    const int t = next_task(V, V.sync + 4 * V.nsn + 1, false, err, phase, &task_id);
-    if (t < 0) break;
-    const SolveTask T = V.tasks[t];
-    const int s = T.s;
-    const int f = V.sn_first[s];
-    const int c = V.sn_first[s + 1] - f;
-    const int64_t rp = V.rows_ptr[s];
-    const int64_t r = V.rows_ptr[s + 1] - rp;
-    const int64_t ld = c + r;
-    const double* P = Lb + V.Lptr[s];
+  sweep_tasks<false, true>(V, M.next, err, [&](int t, int slot, ClaimAhead& next) {
+    const TaskDesc& T = M.next.d[slot];
+    const int s = T.s, f = T.f, c = T.c;
+    const int64_t ld = T.ld;
     const int nr = T.r1 - T.r0;
-    if (nr > 0) load_panel_block_async(M.A, P, c, ld, T.r0, nr);
-    if (T.kind == 0) load_diag_async<false>(M, P, c, ld);
-    if (tid < nr) M.rows[tid] = V.sn_rows[rp + T.r0 + tid];
+    if (nr > 0) load_panel_block_async(M.A, Lb + T.panel, c, ld, nr);
+    if (T.kind == 0) load_diag_async<false>(M, Lb + T.diag, c, ld);
+    if (tid < nr) M.rows[tid] = V.sn_rows[T.rows + tid];
     cp_async_wait_all();
     __syncthreads();
     if (T.kind == 0) finish_diag(M, c);
-    if (!in_queue(V, t)) {  // claimed in order: wait for the inputs, one polling thread each
-      const int q0 = V.tgt_ptr[t], nq = V.tgt_ptr[t + 1] - q0;
-      for (int q = tid; q < nq; q += blockDim.x) wait_geq(xdone + V.tgt[q0 + q], 1, err, 3, spin_limit(V));
-      if (T.kind == 0 && tid == blockDim.x - 1) wait_geq(cdone + s, max(V.nchunk[s], 1) - 1, err, 4, spin_limit(V));
+    if (!in_queue(V, t)) {  // claimed in order: wait for the inputs (one owner: build_sched)
+      if (tid == 0 && T.ntgt > 0) wait_geq(xdone + T.tgt0, 1, err, 3, spin_limit(V));
+      if (T.kind == 0 && tid == blockDim.x - 1) wait_geq(cdone + s, max(T.nchunk, 1) - 1, err, 4, spin_limit(V));
     }
     __syncthreads();
+    next.take();
     // Xr = x[rows] (64 x k); C = L21[rows]^T Xr (c x k)
     double acc[2][NT][2];
     if (nr > 0) load_rows<NT>(M.Y, x, ldx, k, nr, 0, M.rows);
@@ -1599,13 +1573,15 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
       __syncthreads();
       if (tid == 0) {
         atomicAdd(cdone + s, 1);
-        const int d = V.diag_task[s];
-        if (in_queue(V, d) && atomicAdd(V.cnt + d, 1) == V.need[d] - 1) q_push(V, d);
+        if (in_queue(V, t)) {  // its diagonal task follows it in the queue range
+          const int d = V.diag_task[s];
+          if (in_queue(V, d) && atomicAdd(V.cnt + d, 1) == V.need[d] - 1) q_push(V, d);
+        }
       }
     } else {
       // Z = Y_s - (first chunk, here) - (other chunks, accumulated); back-substitute
       store_tile64<NT>(acc, M.A);  // first-chunk products as [j][col]
-      const bool more = V.nchunk[s] > 1;
+      const bool more = T.nchunk > 1;
       __syncthreads();
       constexpr int kB = G::kPer < 16 ? G::kPer : 16;  // loads of a thread in flight
 #pragma unroll
@@ -1635,9 +1611,10 @@ __global__ void __launch_bounds__(kSolveThreads) k_bwd_multi(const SweepView V, 
       __threadfence();
       __syncthreads();
       if (tid == 0) atomicExch(xdone + s, 1);
-      count_owner_done(V, V.dep_ptr[s], V.dep_ptr[s + 1]);  // x_s is out: every queued task whose rows s owns
+      if (V.queue) count_owner_done(V, V.dep_ptr[s], V.dep_ptr[s + 1]);  // x_s is out: every queued task whose rows s owns
     }
-  }
+    next.fetch(V, M.next, slot ^ 1);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -1944,7 +1921,7 @@ void build_sched(const Symbolic& S, int CH, Sched& o, int min_level = 0, int lea
   }
 }
 // Descriptors of the first n tasks of a schedule (see TaskDesc).
-std::vector<TaskDesc> task_descs(const Symbolic& S, const Sched& a, bool forward, const std::vector<int64_t>& dptr) {
+std::vector<TaskDesc> task_descs(const Symbolic& S, const Sched& a, bool forward, const int64_t* dptr) {
   const std::vector<SolveTask>& tasks = forward ? a.ft : a.bt;
   const std::vector<int>&tp = forward ? a.ftp : a.btp, &tg = forward ? a.ftg : a.btg;
   std::vector<TaskDesc> out(forward ? a.nf : a.nb);
@@ -1971,8 +1948,10 @@ std::vector<TaskDesc> task_descs(const Symbolic& S, const Sched& a, bool forward
   return out;
 }
 
-void upload_descs(const Symbolic& S, const Sched& a, const std::vector<int64_t>& dptr, DBuf<TaskDesc>& f,
-                  DBuf<TaskDesc>& b, cudaStream_t st) {
+// dptr: per supernode the offset of its diagonal block as the sweeps read it
+// (the scaled copy, or the block in the panel).
+void upload_descs(const Symbolic& S, const Sched& a, const int64_t* dptr, DBuf<TaskDesc>& f, DBuf<TaskDesc>& b,
+                  cudaStream_t st) {
   const std::vector<TaskDesc> hf = task_descs(S, a, true, dptr), hb = task_descs(S, a, false, dptr);
   f.upload(hf.data(), hf.size(), st);
   b.upload(hb.data(), hb.size(), st);
@@ -2329,7 +2308,7 @@ void upload_tree_plan(temf_ctx& c, int level, int split, bool leaders) {
   T.fexpect.upload(a.expect.data(), a.expect.size(), st);
   T.btgt_ptr.upload(a.btp.data(), a.btp.size(), st);
   T.btgt.upload(a.btg.data(), std::max<size_t>(a.btg.size(), 1), st);
-  upload_descs(S, a, c.fplan.dptr, T.fdesc, T.bdesc, st);
+  upload_descs(S, a, c.fplan.dptr.data(), T.fdesc, T.bdesc, st);
   upload_queue_plan(a, S, split, T.q, st);  // synchronises: the host vectors go out of scope
 }
 
@@ -2375,7 +2354,7 @@ void build_solve_plan(temf_ctx& c) {
   P.nchunk.upload(a.nch.data(), a.nch.size(), st);
   P.part_len = a.poff[nsn];
   P.part_off.upload(a.poff.data(), a.poff.size(), st);
-  upload_descs(S, a, c.fplan.dptr, P.fdesc, P.bdesc, st);
+  upload_descs(S, a, c.fplan.dptr.data(), P.fdesc, P.bdesc, st);
   upload_queue_plan(a, S, default_split(S), P.q1, st);
   TEMF_CUDA(cudaStreamSynchronize(st));  // the host vectors of `a` go out of scope
   upload_multi_plan(c, default_split(S));
@@ -2414,6 +2393,7 @@ void upload_multi_plan(temf_ctx& c, int split) {
   for (int s = 0; s < nsn; ++s) aoff[s + 1] = aoff[s] + (b.nch[s] > 1 ? S.sn_first[s + 1] - S.sn_first[s] : 0);
   P.macc_len = aoff[nsn];
   P.macc_off.upload(aoff.data(), aoff.size(), st);
+  upload_descs(S, b, S.sn_Lptr.data(), P.mfdesc, P.mbdesc, st);
   upload_queue_plan(b, S, split, P.qm, st);  // synchronises: the host vectors go out of scope
 }
 
@@ -2440,6 +2420,10 @@ static int task_grid(K kernel) {
   TEMF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TaskSmem)));
   return persistent_grid(kernel, sizeof(TaskSmem));
 }
+
+// Whether a plan hands any of its tasks out through the ready queue (a queue
+// split at the lowest level leaves none: no queue to clear, seed or look up).
+static bool uses_queue(const QueuePlan& Q, int n_btask) { return Q.f_hi > 0 || Q.b_lo < n_btask; }
 
 static void queued_views(temf_ctx& c, bool block, double* const* Lbase, double* x, SweepView& vf, SweepView& vb);
 static void reset_queues(temf_ctx& c, bool block, cudaStream_t st);
@@ -2496,6 +2480,9 @@ static void queued_views(temf_ctx& c, bool block, double* const* Lbase, double* 
                  block ? P.mnchunk.p : P.nchunk.p, block ? P.macc_off.p : P.part_off.p, c.d_part.p, P.sync.p, P.nsn,
                  nb, q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
                  Q.b_lo, nb, 0, c.spin_limit};
+  vf.desc = block ? P.mfdesc.p : P.fdesc.p;
+  vb.desc = block ? P.mbdesc.p : P.bdesc.p;
+  if (!uses_queue(Q, nb)) vf.queue = vb.queue = nullptr;
 }
 
 // clear the sweep words and seed both queues with their initially ready tasks
@@ -2506,6 +2493,7 @@ static void reset_queues(temf_ctx& c, bool block, cudaStream_t st) {
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;
   TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync_words() * sizeof(int), st));
+  if (!uses_queue(Q, nb)) return;
   TEMF_CUDA(cudaMemsetAsync(q, 0, Q.qbuf.bytes(), st));
   if (Q.n_finit)
     TEMF_CUDA(cudaMemcpyAsync(q, Q.finit.p, Q.n_finit * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -2513,10 +2501,6 @@ static void reset_queues(temf_ctx& c, bool block, cudaStream_t st) {
     TEMF_CUDA(cudaMemcpyAsync(q + nf, Q.binit.p, Q.n_binit * sizeof(int), cudaMemcpyDeviceToDevice, st));
   TEMF_CUDA(cudaMemcpyAsync(words + 2, Q.qtails.p, 2 * sizeof(int), cudaMemcpyDeviceToDevice, st));
 }
-
-// Whether the plan hands any task out through the ready queue (a queue split
-// at the subtree level leaves none: no queue to clear, seed or look up).
-static bool uses_queue(const TreePlan& T) { return T.q.f_hi > 0 || T.q.b_lo < T.n_btask; }
 
 // Views of the single-column sweeps of the tree plan: its task schedules
 // (the supernodes at or above the subtree level) with their ready queue.
@@ -2537,7 +2521,7 @@ static void tree_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& 
                  q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
                  Q.b_lo, nb, 0, c.spin_limit};
   vb.bacc = P.bacc();
-  if (!uses_queue(T)) vf.queue = vb.queue = nullptr;
+  if (!uses_queue(T.q, T.n_btask)) vf.queue = vb.queue = nullptr;
   vf.Dptr = vb.Dptr = F.sn_Dptr.p;
   vf.desc = T.fdesc.p;
   vb.desc = T.bdesc.p;
@@ -2551,7 +2535,7 @@ static void reset_tree_queues(temf_ctx& c, cudaStream_t st) {
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;
   TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync.bytes(), st));  // the sweep words and the column sums
-  if (!uses_queue(T)) return;
+  if (!uses_queue(T.q, T.n_btask)) return;
   TEMF_CUDA(cudaMemsetAsync(q, 0, Q.qbuf.bytes(), st));
   if (Q.n_finit)
     TEMF_CUDA(cudaMemcpyAsync(q, Q.finit.p, Q.n_finit * sizeof(int), cudaMemcpyDeviceToDevice, st));
