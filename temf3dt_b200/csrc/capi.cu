@@ -706,10 +706,16 @@ int temf_spmv(temf_ctx* c, int which, int nrhs, const double* x, double* y, int 
     cudaStream_t st = c->stream;
     for (int q = 0; q < nrhs; ++q)
       TEMF_CUDA(cudaMemcpyAsync(dcol + (size_t)q * n, x + (size_t)q * ld, n * sizeof(double), cudaMemcpyHostToDevice, st));
-    k_permute_in<<<ceil_div((int64_t)vec, 256), 256, 0, st>>>(n, nrhs, perm_dev(c).p, dcol, n, din);
-    launch_spmv(*c, which == 0 ? c->d_M.p : c->d_K.p, din, dout, nrhs, st);
-    k_permute_out<<<ceil_div((int64_t)vec, 256), 256, 0, st>>>(n, nrhs, perm_dev(c).p, dout, n, dcol);
-    TEMF_CHECK_LAUNCH();
+    const double* val = which == 0 ? c->d_M.p : c->d_K.p;
+    if (nrhs == 1) {
+      launch_spmv_user(*c, val, perm_dev(c).p, dcol, dout, st);
+      dcol = dout;
+    } else {
+      k_permute_in<<<ceil_div((int64_t)vec, 256), 256, 0, st>>>(n, nrhs, perm_dev(c).p, dcol, n, din);
+      launch_spmv(*c, val, din, dout, nrhs, st);
+      k_permute_out<<<ceil_div((int64_t)vec, 256), 256, 0, st>>>(n, nrhs, perm_dev(c).p, dout, n, dcol);
+      TEMF_CHECK_LAUNCH();
+    }
     for (int q = 0; q < nrhs; ++q)
       TEMF_CUDA(cudaMemcpyAsync(y + (size_t)q * ld, dcol + (size_t)q * n, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     TEMF_CUDA(cudaStreamSynchronize(st));

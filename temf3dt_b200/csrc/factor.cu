@@ -755,6 +755,7 @@ void build_factor_plan(temf_ctx& c) {
         u.first = (int64_t)tiles.size();
         tiles.insert(tiles.end(), part[k].begin(), part[k].end());
         u.count = (int64_t)tiles.size() - u.first;
+        if (u.count > INT_MAX) throw StateError("too many update tiles in one level");
       }
     }
     F.n_tiles = (int64_t)tiles.size();
@@ -844,7 +845,6 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   TEMF_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(kSnCols)));
   const auto update = [&](const FactorPlan::UpdPart& u, cudaStream_t s) {
     if (u.count == 0) return;
-    if (u.count > INT_MAX) throw StateError("too many update tiles in one level");
     const auto upd = u.shape == kUpdWide ? upd_wide : (u.shape == kUpdDeep ? upd_deep : upd_small);
     const size_t smem = u.shape == kUpdWide ? update_smem<kUpdTile, 2>()
                                             : (u.shape == kUpdDeep ? update_smem<kUpdTile, 4>() : update_smem<kUpdTile / 2, 4>());

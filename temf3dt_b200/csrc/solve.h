@@ -84,6 +84,8 @@ inline size_t two_error_len(int nrhs) { return (size_t)(1 + 296) * 2 * nrhs; }
 void launch_two_error(temf_ctx& c, const double* a, const double* b, int nrhs, double* out, cudaStream_t st);
 // plain y = M x (full symmetric)
 void launch_spmv(temf_ctx& c, const double* M, const double* x, double* y, int nrhs, cudaStream_t st);
+// the same for one column in the original numbering (perm: device, perm[new] = old)
+void launch_spmv_user(temf_ctx& c, const double* M, const int* perm, const double* x, double* y, cudaStream_t st);
 
 // Many models at once: views of one model's sweeps (the forward view carries
 // the forward schedule, the backward view the backward one; `sync` is that
