@@ -333,8 +333,9 @@ int temf_symbolic_host(int n, const long long* xadj, const int* adj, const doubl
                        double* stats);
 
 /* Host-only check of an analysis (no GPU needed): the supernode row lists (ascending, below the diagonal block, every child row
- * inside its parent's panel), then the triangular-solve schedules replayed,
- * claimed in order and through the ready queue, for both chunk heights.
+ * inside its parent's panel), the levels whose factor updates may run side by
+ * side, then the triangular-solve schedules replayed, claimed in order and
+ * through the ready queue, for both chunk heights.
  * Returns 0, or 1 with the first violation in msg. */
 int temf_schedule_check(int n, const long long* xadj, const int* adj, const double* xyz, char* msg, int msg_len);
 

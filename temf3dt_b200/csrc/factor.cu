@@ -419,7 +419,6 @@ __device__ __forceinline__ void mbar_wait(uint64_t* b, unsigned parity, int* err
 // and a read-modify-write scatter, 49 as 32 x 32 tiles).  An entry's sum runs
 // over the same columns in the same order in every shape.
 constexpr int kUpdChunk = 16;
-constexpr int kUpdMaxMembers = 8;
 
 template <int kT, int kStages>
 constexpr size_t update_smem() {
@@ -592,24 +591,6 @@ inline UpdShape update_shape(int64_t tiles64) {
 // ---------------------------------------------------------------------------
 // host plan
 // ---------------------------------------------------------------------------
-// Runs of the factor's Schur updates: up to `max_members` consecutive
-// supernodes that are the column blocks of one wider supernode -- each the
-// parent of the previous, and each one's rows exactly the next block's
-// columns followed by the next block's rows.  run_end[s] = the last member
-// of s's run (s itself outside runs).
-std::vector<int> update_runs(const Symbolic& S, int max_members) {
-  const int nsn = S.nsn;
-  const std::vector<int> run_first = block_run_first(S);
-  std::vector<int> end(nsn);
-  for (int s = 0; s < nsn;) {
-    int e = s;
-    while (e - s + 1 < max_members && e + 1 < nsn && run_first[e + 1] == run_first[s]) ++e;
-    for (int q = s; q <= e; ++q) end[q] = e;
-    s = e + 1;
-  }
-  return end;
-}
-
 void build_factor_plan(temf_ctx& c) {
   const Symbolic& S = c.sym;
   FactorPlan& F = c.fplan;
@@ -724,7 +705,10 @@ void build_factor_plan(temf_ctx& c) {
     };
     // A level's tiles in two parts: those with a column of the next level's
     // supernodes (the next level waits for them), then the others (by the 64
-    // columns a tile lies in, whatever its own size).
+    // columns a tile lies in, whatever its own size).  One part where supernodes
+    // of the level update entries in common: two parts run side by side, and the
+    // one that arrives first decides the rounding of such an entry's sum.
+    const std::vector<char> apart = levels_apart(S, run_end);
     int flagged = -1;  // supernode of `flags`: per 64 columns, whether they hold one
     std::vector<char> flags;
     auto urgent = [&](const UpdTile& t, int l) {
@@ -742,7 +726,7 @@ void build_factor_plan(temf_ctx& c) {
     for (int l = 0; l < S.nlevels; ++l) {
       std::vector<UpdTile> all, small, part[2];
       level_tiles(l, kUpdTile, all, true);
-      for (const UpdTile& t : all) part[urgent(t, l) ? 0 : 1].push_back(t);
+      for (const UpdTile& t : all) part[!apart[l] || urgent(t, l) ? 0 : 1].push_back(t);
       for (int k = 0; k < 2; ++k) {
         FactorPlan::UpdPart& u = F.upd[2 * l + k];
         u.shape = update_shape((int64_t)part[k].size());
@@ -750,7 +734,7 @@ void build_factor_plan(temf_ctx& c) {
           if (small.empty()) level_tiles(l, kUpdTile / 2, small, false);
           part[k].clear();
           for (const UpdTile& t : small)
-            if (urgent(t, l) == (k == 0)) part[k].push_back(t);
+            if ((!apart[l] || urgent(t, l)) == (k == 0)) part[k].push_back(t);
         }
         u.first = (int64_t)tiles.size();
         tiles.insert(tiles.end(), part[k].begin(), part[k].end());
@@ -857,8 +841,9 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   // the next level waits for) runs on a high-priority stream, the level's
   // other updates on the context's stream, behind the next level's blocks and
   // row solves (one CTA and a few, about 30 us).  A level's urgent updates
-  // wait for the other updates of the level before: every entry receives its
-  // levels' sums in the order of one stream.
+  // wait for the other updates of the level before, and the two parts of a
+  // level have no entry in common (levels_apart): every entry receives its
+  // sums as in one stream.
   FactorStreams& W = c.fac;
   W.ensure();
   const cudaStream_t hi = W.chain;

@@ -511,6 +511,62 @@ std::string check_update_groups(const Symbolic& S) {
   return std::string();
 }
 
+std::vector<int> update_runs(const Symbolic& S, int max_members) {
+  const int nsn = S.nsn;
+  const std::vector<int> run_first = block_run_first(S);
+  std::vector<int> end(nsn);
+  for (int s = 0; s < nsn;) {
+    int e = s;
+    while (e - s + 1 < max_members && e + 1 < nsn && run_first[e + 1] == run_first[s]) ++e;
+    for (int q = s; q <= e; ++q) end[q] = e;
+    s = e + 1;
+  }
+  return end;
+}
+
+// Columns that the updates of s reach: the later members' of its run, or all its rows.
+static int update_cols(const Symbolic& S, const std::vector<int>& run_end, int s) {
+  const int e = run_end[s];
+  return e != s ? S.sn_first[e + 1] - S.sn_first[s + 1] : (int)(S.sn_rows_ptr[s + 1] - S.sn_rows_ptr[s]);
+}
+
+std::vector<char> levels_apart(const Symbolic& S, const std::vector<int>& run_end) {
+  std::vector<char> apart(S.nlevels, 1);
+  std::vector<int> level_of(S.n, -1);  // per column: the last level that updates it
+  for (int l = 0; l < S.nlevels; ++l) {
+    for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1] && apart[l]; ++q) {
+      const int s = S.level_sn[q];
+      const int* rows = S.sn_rows.data() + S.sn_rows_ptr[s];
+      const int n = update_cols(S, run_end, s);
+      for (int k = 0; k < n; ++k) {
+        if (level_of[rows[k]] == l) apart[l] = 0;  // two updates of a column share its diagonal entry
+        level_of[rows[k]] = l;
+      }
+    }
+  }
+  return apart;
+}
+
+std::string check_levels_apart(const Symbolic& S) {
+  const std::vector<int> run_end = update_runs(S, kUpdMaxMembers);
+  const std::vector<char> apart = levels_apart(S, run_end);
+  for (int l = 0; l < S.nlevels; ++l) {
+    if (!apart[l]) continue;
+    std::vector<int64_t> entries;  // all that the level updates
+    for (int q = S.level_ptr[l]; q < S.level_ptr[l + 1]; ++q) {
+      const int s = S.level_sn[q];
+      const int* rows = S.sn_rows.data() + S.sn_rows_ptr[s];
+      const int r = (int)(S.sn_rows_ptr[s + 1] - S.sn_rows_ptr[s]), n = update_cols(S, run_end, s);
+      for (int j = 0; j < n; ++j)
+        for (int i = j; i < r; ++i) entries.push_back((int64_t)rows[j] * S.n + rows[i]);
+    }
+    std::sort(entries.begin(), entries.end());
+    if (std::adjacent_find(entries.begin(), entries.end()) != entries.end())
+      return "level " + std::to_string(l) + " counts as free of common entries and is not";
+  }
+  return std::string();
+}
+
 std::vector<int> nested_dissection(int n, const int64_t* xadj, const int* adj,
                                    const double* xyz, int leaf_size, int threads) {
   NDState S;

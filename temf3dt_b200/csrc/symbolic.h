@@ -96,6 +96,20 @@ void update_groups(const Symbolic& S, UpdateGroups& G, int threads = 0);
 // lands on that row of its target panel.  Empty string, or the violation.
 std::string check_update_groups(const Symbolic& S);
 
+// Runs of the factor's Schur updates: up to `max_members` consecutive
+// supernodes that are the column blocks of one wider supernode -- each the
+// parent of the previous, and each one's rows exactly the next block's
+// columns followed by the next block's rows.  run_end[s] = the last member
+// of s's run (s itself outside runs).
+constexpr int kUpdMaxMembers = 8;
+std::vector<int> update_runs(const Symbolic& S, int max_members);
+
+// Per level: whether no two of its supernodes update an entry in common, so
+// that its updates may run side by side in any order without a sum changing.
+std::vector<char> levels_apart(const Symbolic& S, const std::vector<int>& run_end);
+// Host check of the levels found apart, entry by entry.  Empty string, or the violation.
+std::string check_levels_apart(const Symbolic& S);
+
 // Host threads to use for a request (0: $TEMF_HOST_THREADS, else the cores
 // this process may run on, bounded by the cgroup CPU quota, at most 64).
 int host_threads(int requested);

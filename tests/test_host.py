@@ -218,6 +218,22 @@ def test_solve_schedules_replay(kind):
     assert rc == 0, msg.value.decode()
 
 
+@pytest.mark.parametrize("kind", ["slab", "cube", "mesh"])
+def test_factor_updates_side_by_side_share_no_entry(kind):
+    """A level's factor updates run in two launches side by side only where no
+    two of its supernodes update an entry in common (checked entry by entry):
+    which launch comes first then changes no sum."""
+    if kind == "mesh":
+        from tests.golden_cases import tiny_synth
+        n, xadj, adj, xyz = _edge_pattern(tiny_synth())
+    else:
+        n, xadj, adj, xyz = _grid_pattern(*((40, 30, 4) if kind == "slab" else (17, 16, 15)))
+    msg = C.create_string_buffer(256)
+    rc = _lib.lib().temf_schedule_check(n, xadj.ctypes.data_as(C.POINTER(C.c_longlong)), _lib.iptr(adj),
+                                        _lib.dptr(xyz), msg, 256)
+    assert rc == 0, msg.value.decode()
+
+
 def test_ordering_does_not_depend_on_host_threads(monkeypatch):
     """The nested-dissection halves and the three axis evaluations of large
     subsets run on separate host threads; the permutation and the symbolic
