@@ -339,6 +339,11 @@ int temf_symbolic_host(int n, const long long* xadj, const int* adj, const doubl
  * Returns 0, or 1 with the first violation in msg. */
 int temf_schedule_check(int n, const long long* xadj, const int* adj, const double* xyz, char* msg, int msg_len);
 
+/* The arithmetic that the factor's rounding rests on, on the context's device.
+ * which 0: out[i] = a[i] / b[i] as the row solves divide (n values each).
+ * which 1: n tiles out (8 x 8, row-major) += a (8 x 4) b (4 x 8) as one DMMA. */
+int temf_arith_check(temf_ctx* ctx, int which, int n, const double* a, const double* b, double* out);
+
 /* ---- PARDISO-compatible shim ------------------------------------------------
  * Same argument meaning as the reference's module pardiso_multi_real_mpi
  * (src/FETD_UTILITY.f90:826-1028) so adap_euler can keep its five calls.

@@ -37,6 +37,7 @@ SIGNATURES = {
     "temf_solve": (_i, [_p, _i, _i, _dp, _dp, _i]),
     "temf_release": (_i, [_p, _i]),
     "temf_solve_noalloc": (_i, [_p, _i, _p, _p]),
+    "temf_arith_check": (_i, [_p, _i, _i, _dp, _dp, _dp]),
     "temf_spmv": (_i, [_p, _i, _i, _dp, _dp, _i]),
     "temf_set_sources": (_i, [_p, _i, _ip, _ip, _ip, _i, _i, _d, _d]),
     "temf_set_receivers": (_i, [_p, _i, _ip, _dp, _ip]),

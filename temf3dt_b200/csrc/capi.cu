@@ -1329,6 +1329,14 @@ int temf_schedule_check(int n, const long long* xadj, const int* adj, const doub
   }
 }
 
+int temf_arith_check(temf_ctx* c, int which, int n, const double* a, const double* b, double* out) {
+  return guarded(c, [&] {
+    if ((which != 0 && which != 1) || n < 1 || !a || !b || !out) throw ArgError("temf_arith_check: bad arguments");
+    arith_check(which, n, a, b, out);
+    return TEMF_OK;
+  });
+}
+
 // ---- PARDISO shim -----------------------------------------------------------
 }  // extern "C"
 

@@ -237,12 +237,21 @@ __global__ void __launch_bounds__(kPotrfThreads, 2) k_potrf(
 // corrections of a y, the last of which rounds correctly (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
 // processor", IBM J. Res. Dev. 34, 1990, theorem on quotients) while neither
-// over- nor underflows.  45 cycles on the chain of a row, a division 110.
+// over- nor underflows: b one that divisor_fits() takes, the result finite and
+// its quotient_key() at least kQuotientKey (a - q b is a double then).  The
+// caller divides otherwise.  45 cycles on the chain of a row, a division 110.
 __device__ __forceinline__ double quotient(double a, double b, double y) {
   double q = a * y;
-  q = fma(fma(-q, b, a), y, q);
-  return fma(fma(-q, b, a), y, q);
+  q = fma(-fma(q, b, -a), y, q);  // (in this form a zero keeps its sign)
+  return fma(-fma(q, b, -a), y, q);
 }
+// square roots of positive doubles; not the infinite one, not NaN
+__device__ __forceinline__ bool divisor_fits(double b) { return b >= 0x1p-537 && b <= 0x1p512; }
+// grows with |q|, zeros on top: kQuotientKey for 2^-400
+__device__ __forceinline__ unsigned quotient_key(double q) {
+  return ((unsigned)__double2hiint(q) & 0x7fffffffu) - 1u + min((unsigned)__double2loint(q), 1u);
+}
+constexpr unsigned kQuotientKey = ((1023u - 400u) << 20) - 1u;
 
 // Below-diagonal rows of the level's supernodes, kTrsmRows rows per CTA:
 // x L11^T = a, L21 = x S11 in the indefinite mode (sgn != null).  Panels of 16
@@ -263,6 +272,15 @@ constexpr int kLdX = kTrsmRows + 4;         // DMMA fragments (4 columns x 8 row
 inline size_t trsm_smem(int width) {        // X [w][kLdX], the block [w][kLdD], 1 / L_kk [w]; w: whole panels
   const int w = (width + kTrsmPanel - 1) / kTrsmPanel * kTrsmPanel;
   return (size_t)w * (kLdX + kLdD + 1) * sizeof(double);
+}
+
+// One row of a panel with divisions: infinities, NaN, values at the ends of the range.
+__device__ __noinline__ void divide_panel(double* x, const double* D) {
+  for (int j = 0; j < kTrsmPanel; ++j) {
+    const double v = x[j * kLdX] / D[j * kLdD + j];
+    x[j * kLdX] = v;
+    for (int k = j + 1; k < kTrsmPanel; ++k) x[k * kLdX] -= v * D[k * kLdD + j];
+  }
 }
 
 __global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restrict__ chunks,
@@ -296,7 +314,7 @@ __global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restri
   }
   __syncthreads();
   if (tid < w) rinv[tid] = 1.0 / D[tid * kLdD + tid];
-  __syncthreads();
+  const bool fits = __syncthreads_and(tid >= w || divisor_fits(D[tid * kLdD + tid]));
   for (int p = 0; p < np; ++p) {
     const int j0 = kTrsmPanel * p;
     if (p > 0) {  // rows 16 warp .. + 15 of the panel minus the products with the columns before it
@@ -337,6 +355,15 @@ __global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restri
 #pragma unroll
         for (int k = j + 1; k < kTrsmPanel; ++k) x[k] -= x[j] * D[(j0 + k) * kLdD + j0 + j];
       }
+      unsigned key = ~0u;
+#pragma unroll
+      for (int j = 0; j < kTrsmPanel; ++j) key = min(key, quotient_key(x[j]));
+      // what is not finite has made the last column NaN
+      if (!fits || key < kQuotientKey || !isfinite(x[kTrsmPanel - 1])) {
+        divide_panel(X + j0 * kLdX + t, D + j0 * kLdD + j0);
+#pragma unroll
+        for (int j = 0; j < kTrsmPanel; ++j) x[j] = X[(j0 + j) * kLdX + t];
+      }
 #pragma unroll
       for (int j = 0; j < kTrsmPanel; ++j) {
         X[(j0 + j) * kLdX + t] = x[j];
@@ -345,6 +372,39 @@ __global__ void __launch_bounds__(kTrsmThreads) k_trsm(const TrsmChunk* __restri
     }
     __syncthreads();
   }
+}
+
+// The arithmetic that the factor's rounding rests on, one operand set per
+// thread or warp (temf_arith_check).
+__global__ void k_check_quotient(int n, const double* __restrict__ a, const double* __restrict__ b,
+                                 double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double q = quotient(a[i], b[i], 1.0 / b[i]);
+  out[i] = divisor_fits(b[i]) && quotient_key(q) >= kQuotientKey && isfinite(q) ? q : a[i] / b[i];
+}
+__global__ void k_check_dmma(int n, const double* __restrict__ a, const double* __restrict__ b,
+                             double* __restrict__ out) {
+  const int t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32);
+  if (t >= n) return;  // whole warps
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  double* c = out + 64 * (size_t)t + 8 * g + 2 * q;
+  double c0 = c[0], c1 = c[1];
+  dmma_8x8x4(c0, c1, a[32 * (size_t)t + 4 * g + q], b[32 * (size_t)t + 8 * q + g]);
+  c[0] = c0;
+  c[1] = c1;
+}
+
+void arith_check(int which, int n, const double* a, const double* b, double* out) {
+  const size_t in = which == 0 ? n : 32 * (size_t)n, res = which == 0 ? n : 64 * (size_t)n;
+  DBuf<double> da, db, dc;
+  da.upload(a, in, 0);
+  db.upload(b, in, 0);
+  dc.upload(out, res, 0);
+  if (which == 0) k_check_quotient<<<ceil_div(n, 256), 256>>>(n, da.p, db.p, dc.p);
+  else k_check_dmma<<<ceil_div(32 * (int64_t)n, 256), 256>>>(n, da.p, db.p, dc.p);
+  TEMF_CHECK_LAUNCH();
+  TEMF_CUDA(cudaMemcpy(out, dc.p, res * sizeof(double), cudaMemcpyDeviceToHost));
 }
 
 // Bulk global -> shared copies on the TMA engine (cp.async.bulk, this GPU's

@@ -27,4 +27,6 @@ int finish_factor(temf_ctx& c, int slot);
 // non-positive pivot column (original numbering, 1-based) with a valid
 // indefinite factor.
 int numeric_factor_values_fallback(temf_ctx& c, int slot, const double* X, double a, const double* Y, double b);
+// The factor's own arithmetic on given operands: see temf_arith_check.
+void arith_check(int which, int n, const double* a, const double* b, double* out);
 }  // namespace temf

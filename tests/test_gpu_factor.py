@@ -1,12 +1,15 @@
 """The factor's kernels at the widths and row counts where they can go wrong:
 analysis options move the supernode widths over the elimination panels and
 the tile edges, and a planted pivot is found wherever it stands in its block.
-Backward error 1e-12, the bound of the other solves."""
+Backward error 1e-12, the bound of the other solves.  The arithmetic that the
+factor's rounding rests on, to the bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
 
-from temf3dt_b200 import fetd
+from temf3dt_b200 import _lib, fetd
 from tests.golden_cases import tiny_synth
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +59,74 @@ def test_planted_pivot_is_found_in_every_position():
             va = U.data.copy()
             va[ia[col] - 1] = -10.0 * abs(va[ia[col] - 1])    # the diagonal is a row's first entry
             assert g.pardiso_direct_1(1, ia, ja, va) == col + 1
+
+
+def test_infinite_diagonal_fixes_its_unknown():
+    """An infinite diagonal entry (a Dirichlet condition as a penalty without
+    end) gives x = 0 there and the reduced system's solution elsewhere: the
+    rows below it are zero (finite / inf), not NaN."""
+    m = tiny_synth()
+    with _context(m, 96, 2) as g:
+        ia, ja, U, A = _matrix(g, 1e-6)
+        g.pardiso_alloc(2)
+        rng = np.random.default_rng(1)
+        fixed = rng.choice(g.n_edges, 7, replace=False)
+        va = U.data.copy()
+        va[ia[fixed] - 1] = np.inf
+        assert g.pardiso_direct_1(1, ia, ja, va) == 0
+        free = np.setdiff1d(np.arange(g.n_edges), fixed)
+        R = A[free][:, free]
+        for cols in (1, 3):
+            b = rng.standard_normal((g.n_edges, cols))
+            b[free] = R @ b[free]
+            x = g.solve(1, b[:, 0] if cols == 1 else b).reshape(g.n_edges, cols)
+            assert np.all(x[fixed] == 0.0)
+            r = np.linalg.norm(R @ x[free] - b[free], axis=0) / np.linalg.norm(b[free], axis=0)
+            assert r.max() <= 1e-12
+
+
+def _arith(which, n, a, b, out):
+    m = tiny_synth()
+    with _context(m, 96, 2) as g:
+        a, b, out = (np.ascontiguousarray(v, dtype=np.float64) for v in (a, b, out))
+        g._ck(_lib.lib().temf_arith_check(g._h, which, n, _lib.dptr(a), _lib.dptr(b), _lib.dptr(out)), "temf_arith_check")
+        return out
+
+
+def test_row_solves_divide_as_the_division_does():
+    """Bit for bit, over operands of full mantissas and over those where a
+    corrected reciprocal product is hardest: mantissas next to 1 and 2, exact
+    quotients, quotients next to a midpoint of two doubles; exponents up to
+    the ends of a factor's diagonal and past the range of the corrections;
+    zeros of both signs, infinities and NaN."""
+    rng = np.random.default_rng(0)
+    n = 1 << 19
+
+    def mantissas(k):
+        m = 1.0 + rng.random(k)
+        e = rng.integers(0, 4, k) * 2.0 ** -52
+        return np.where(rng.random(k) < 0.2, np.where(rng.random(k) < 0.5, 1.0 + e, 2.0 - 2.0 ** -52 - e), m)
+
+    a, b = [], []
+    for lo, hi in ((-30, 30), (-500, 500)):                   # L_kk = sqrt(d): 2^-537 to 2^512
+        den = np.ldexp(mantissas(n), rng.integers(lo, hi, n))
+        q = mantissas(n)
+        top = np.where(rng.random(n) < 0.4, q * den,          # next to an exact quotient
+                       np.where(rng.random(n) < 0.5, q * den + 0.5 * np.spacing(q) * den, mantissas(n) * den))
+        a.append(top * np.where(rng.random(n) < 0.5, 1.0, -1.0))
+        b.append(den)
+    den = np.ldexp(mantissas(n), rng.integers(-537, 512, n))
+    a.append(np.ldexp(mantissas(n), rng.integers(-1074, 1023, n)))  # all exponents, denormal to the largest
+    b.append(den)
+    k = rng.integers(1, 1 << 26, (2, n)).astype(np.float64)   # exact quotients
+    a.append(k[0] * k[1])
+    b.append(k[1])
+    special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 1e308, 1.0])
+    a.append(np.repeat(special, 5))
+    b.append(np.tile([np.inf, np.nan, 1.0, 2.0 ** 512, 2.0 ** -537], len(special)))
+    a, b = np.concatenate(a), np.concatenate(b)
+    got = _arith(0, len(a), a, b, np.zeros(len(a)))
+    with np.errstate(all="ignore"):
+        want = a / b
+    same = (got.view(np.uint64) == want.view(np.uint64)) | (np.isnan(got) & np.isnan(want))
+    assert same.all(), (a[~same][:4], b[~same][:4], got[~same][:4], want[~same][:4])
