@@ -130,3 +130,48 @@ def test_row_solves_divide_as_the_division_does():
         want = a / b
     same = (got.view(np.uint64) == want.view(np.uint64)) | (np.isnan(got) & np.isnan(want))
     assert same.all(), (a[~same][:4], b[~same][:4], got[~same][:4], want[~same][:4])
+
+
+def test_dmma_adds_its_products_in_ascending_order():
+    """The tiles of the blocks' elimination and of the row solves keep the
+    rounding of column-by-column elimination: a DMMA with the target as the
+    accumulator is four FMAs, one after the other in ascending k."""
+    fma = C.CDLL("libm.so.6").fma
+    fma.restype, fma.argtypes = C.c_double, [C.c_double] * 3
+    rng = np.random.default_rng(0)
+    n = 256
+    scale = lambda shape: np.ldexp(rng.standard_normal(shape), rng.integers(-20, 20, shape))
+    a, b, c = scale((n, 8, 4)), scale((n, 4, 8)), scale((n, 8, 8))
+    got = _arith(1, n, a, b, c.copy()).reshape(n, 8, 8)
+    for t in range(n):
+        for i in range(8):
+            for j in range(8):
+                v = c[t, i, j]
+                for k in range(4):
+                    v = fma(a[t, i, k], b[t, k, j], v)
+                assert v == got[t, i, j]
+
+
+def test_planted_pivot_is_found_at_every_offset_of_a_block():
+    """Each of the last 130 columns in elimination order: every position of at
+    least one whole 64-column block, in every elimination panel."""
+    m = tiny_synth()
+    with _context(m, 96, 2) as g:
+        ia, ja, U, A = _matrix(g, 1e-6)
+        P = A.tocsr()
+        P.sort_indices()
+        n = g.n_edges
+        off = P.indices != np.repeat(np.arange(n), np.diff(P.indptr))
+        xadj = np.concatenate([[0], np.cumsum(np.add.reduceat(off, P.indptr[:-1]))]).astype(np.int64)
+        adj = P.indices[off].astype(np.int32)
+        nod, edg = m.mesh.nod_cor, fetd.mesh_topology(m.mesh.tet_vex)[0]
+        mid = np.ascontiguousarray(0.5 * (nod[edg[:, 0] - 1] + nod[edg[:, 1] - 1]))
+        perm, st = np.zeros(n, dtype=np.int32), np.zeros(9)
+        assert _lib.lib().temf_symbolic_host(n, xadj.ctypes.data_as(C.POINTER(C.c_longlong)), _lib.iptr(adj),
+                                             _lib.dptr(mid), _lib.iptr(perm), _lib.dptr(st)) == 0
+        assert st[1] == g.stats()["supernodes"]               # the same analysis as the context's
+        g.pardiso_alloc(2)
+        for col in perm[-130:]:
+            va = U.data.copy()
+            va[ia[col] - 1] = -10.0 * abs(va[ia[col] - 1])
+            assert g.pardiso_direct_1(1, ia, ja, va) == col + 1
