@@ -232,7 +232,7 @@ void run_adjoint(temf_ctx& c, const double* dJ, int rows, const int* tet_cell, i
       TEMF_CUDA(cudaEventElapsedTime(&ms, f0, f1));
       res.ms_factor += ms;
       res.n_factor += 1;
-      res.launches += 2 + 2 * (int64_t)c.sym.nlevels;
+      res.launches += factor_launch_count(c);
       if (stt != 0) throw StateError("non-positive pivot in the adjoint factorisation");
       cur_dt = dt;
     }
@@ -245,7 +245,7 @@ void run_adjoint(temf_ctx& c, const double* dJ, int rows, const int* tet_cell, i
       res.launches += 1;
       if (A.coef[j - 1] != 0.0) { launch_source(c, d_coef.p + (j - 1), X(j), 1, st); res.launches += 1; }
       launch_solve(c, lp.p, X(j), 1, st);
-      res.launches += 2;
+      res.launches += solve_launch_count(c, 1);
     }
     for (int k = e - 1; k >= f; --k) {
       const double* pa = vecsum(kid_a[k], va);
@@ -260,7 +260,7 @@ void run_adjoint(temf_ctx& c, const double* dJ, int rows, const int* tet_cell, i
         res.launches += 1;
       }
       launch_solve(c, lp.p, lk, 1, st);
-      res.launches += 2;
+      res.launches += solve_launch_count(c, 1);
       k_grad_tets<<<ceil_div(T, 128), 128, 0, st>>>(T, d_te.p, d_Mu.p, lk, X(k), X(A.a[k - 1]), X(A.b[k - 1]),
                                                      d_G.p);
       TEMF_CHECK_LAUNCH();

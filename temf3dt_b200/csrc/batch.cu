@@ -367,7 +367,7 @@ struct BatchEngine {
     for (auto& j : jobs) {
       const int stt = finish_factor(*j.first->c, j.second.first);
       j.first->res->n_factor += 1;
-      S.launches += 2 + 2 * (int64_t)j.first->c->sym.nlevels;
+      S.launches += factor_launch_count(*j.first->c);
       if (stt != 0)
         throw StateError("non-positive pivot in a batched step-matrix factorisation at column " + std::to_string(stt));
     }

@@ -851,6 +851,15 @@ int finish_factor(temf_ctx& c, int slot) {
   return 0;
 }
 
+int64_t factor_launch_count(const temf_ctx& c) {
+  const FactorPlan& F = c.fplan;
+  int64_t n = F.n_a2l > 0 ? 1 : 0;
+  for (int l = 0; l < c.sym.nlevels; ++l)
+    n += (c.sym.level_ptr[l + 1] > c.sym.level_ptr[l]) + (F.trsm_level_ptr[l + 1] > F.trsm_level_ptr[l]) +
+         (F.upd[2 * l].count > 0) + (F.upd[2 * l + 1].count > 0);
+  return n;
+}
+
 void launch_factor(temf_ctx& c, int slot, double dt) {
   launch_factor_values(c, slot, c.d_M.p, 3.0, c.d_K.p, 2.0 * dt);
 }

@@ -22,6 +22,8 @@ void launch_factor(temf_ctx& c, int slot, double dt);
 void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, const double* Y, double b,
                           bool indefinite = false);
 int finish_factor(temf_ctx& c, int slot);
+// kernels of one factorisation
+int64_t factor_launch_count(const temf_ctx& c);
 // numeric_factor_values, and when A is not positive definite the indefinite
 // factorisation into the same slot: returns 0 (LL^T) or the first
 // non-positive pivot column (original numbering, 1-based) with a valid

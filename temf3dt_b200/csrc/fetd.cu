@@ -241,7 +241,7 @@ struct Engine {
     TEMF_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
     res.ms_factor += ms;
     res.n_factor += 1;
-    res.launches += 2 + 2 * (int64_t)c.sym.nlevels;
+    res.launches += factor_launch_count(c);
     if (stt != 0)
       throw StateError("non-positive pivot in the step-matrix factorisation at column " + std::to_string(stt) +
                        " (dt = " + std::to_string(dt) + ")");
