@@ -2387,7 +2387,14 @@ void build_solve_plan(temf_ctx& c) {
   // leaders, 150k 0.86 against 2.0, 1.48M 6.1 against 11.5).
   const int level = default_tree_level(S);
   upload_tree_plan(c, level, level, false);
+  // an earlier analysis's tuning says nothing about this one
   P.tree.tuned = false;
+  P.tree.tune_level.clear();
+  for (QueuePlan* Q : {&P.q1, &P.qm, &P.tree.q}) {
+    Q->tuned = false;
+    Q->tune_ms.clear();
+    Q->tune_split.clear();
+  }
   TEMF_CUDA(cudaStreamSynchronize(st));
 }
 

@@ -6,7 +6,8 @@ Backward error 1e-12, the bound of the other solves."""
 import numpy as np
 import pytest
 
-from tests.golden_cases import tiny_synth
+from temf3dt_b200 import fetd
+from tests.golden_cases import small_synth, tiny_synth
 from tests.test_gpu_factor import _context, _matrix
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +40,28 @@ def test_single_column_plans(factored, level, split, leaders):
     b = A @ np.random.default_rng(split).standard_normal(g.n_edges)
     for _ in range(2):
         assert _worst(A, g.solve(1, b)[:, None], b[:, None]) <= 1e-12
+
+
+def test_a_new_analysis_is_untuned():
+    """What was tuned on one mesh does not stand for the next one in the same
+    context, for one column or for several."""
+    with _context(tiny_synth(), 96, 2) as g:
+        assert g.factor(1, 2e-6) == 0
+        for cols in (1, 5):
+            g.tune_solve(1, cols)
+            assert g.solve_schedule(cols)[1]
+        m = small_synth()
+        edg, te, td = fetd.mesh_topology(m.mesh.tet_vex)
+        g.set_mesh(m.mesh.nod_cor, m.mesh.tet_vex, edg, te, td)
+        g.set_media(*fetd.meshio.media_per_tet(m.mesh.tet_phy, m.ctl))
+        g.set_boundary(0)
+        g.analyse()
+        assert not g.solve_schedule(1)[1] and not g.solve_schedule(5)[1] and not g.solve_plan()["tuned"]
+        g.assemble()
+        assert g.factor(1, 2e-6) == 0
+        A = _matrix(g, 2e-6)[3]
+        for cols in (1, 5):
+            b = A @ np.random.default_rng(cols).standard_normal((g.n_edges, cols))
+            assert _worst(A, g.solve(1, b).reshape(b.shape), b) <= 1e-12
+            g.tune_solve(1, cols)
+            assert g.solve_schedule(cols)[1]
