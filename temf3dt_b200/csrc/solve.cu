@@ -777,36 +777,12 @@ __device__ void bwd_leader(const SweepView& V, int t, const double* Lb, int* err
       bwd_row_sums(R, zi, seg);
       __syncthreads();
     }
-    // z = y_q - (first chunk) - (other chunks, fixed order)
-    const int nch = V.nchunk[q];
-    const double* pp = V.part + V.part_off[q];
-    double* psum = &M.rows[0][0];  // [2][64]
-    if (nch > 1 && V.bacc) {
-      for (int j = tid; j < c; j += blockDim.x) {
-        psum[j] = __ldcg(V.bacc + f + j);
-        psum[kSnCols + j] = 0.0;
-      }
-      __syncthreads();
-    } else if (nch > 1) {
-      const int j = tid & (kSnCols - 1), h = tid / kSnCols;
-      double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (j < c && h < 2) {
-        int k = 1 + h;
-        for (; k + 14 < nch; k += 16) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) acc[u] += __ldcg(pp + (int64_t)(k + 2 * u) * c + j);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (k + 2 * u < nch) acc[u] += __ldcg(pp + (int64_t)(k + 2 * u) * c + j);
-      }
-      if (h < 2) psum[h * kSnCols + j] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-      __syncthreads();
-    }
+    // z = y_q - (first chunk) - (column sums of the other chunks)
+    const bool more = V.nchunk[q] > 1;
     for (int j = tid; j < c; j += blockDim.x) {
       double v = __ldcg(x + f + j);
       if (r1 > 0) v -= (seg[0][j] + seg[1][j]) + (seg[2][j] + seg[3][j]);
-      if (nch > 1) v -= psum[j] + psum[kSnCols + j];
+      if (more) v -= __ldcg(V.bacc + f + j);
       M.ys[j] = v;
     }
     if (tid >= c && tid < kSnCols) M.ys[tid] = 0.0;
@@ -2453,8 +2429,8 @@ static int task_grid(K kernel) {
 // split at the lowest level leaves none: no queue to clear, seed or look up).
 static bool uses_queue(const QueuePlan& Q, int n_btask) { return Q.f_hi > 0 || Q.b_lo < n_btask; }
 
-static void queued_views(temf_ctx& c, bool block, double* const* Lbase, double* x, SweepView& vf, SweepView& vb);
-static void reset_queues(temf_ctx& c, bool block, cudaStream_t st);
+static void block_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& vf, SweepView& vb);
+static void reset_block_queues(temf_ctx& c, cudaStream_t st);
 
 static void scale_rows(temf_ctx& c, const double* sgn, double* x, int ld, int ncol, cudaStream_t st);
 
@@ -2471,8 +2447,8 @@ static void launch_solve_multi(temf_ctx& c, double* const* Lbase, double* x, int
     const int gridf = std::min(persistent_grid(fwd, smem), std::max(P.n_mftask, 1));
     const int gridb = std::min(persistent_grid(bwd, smem), std::max(P.n_mbtask, 1));
     SweepView vf, vb;
-    queued_views(c, true, Lbase, x + c0, vf, vb);
-    reset_queues(c, true, st);
+    block_views(c, Lbase, x + c0, vf, vb);
+    reset_block_queues(c, st);
     fwd<<<gridf, kSolveThreads, smem, st>>>(vf, nrhs, k, c.d_status.p + 1);
     TEMF_CHECK_LAUNCH();
     if (sgn) scale_rows(c, sgn, x + c0, nrhs, k, st);  // indefinite factor: L S L^T
@@ -2488,36 +2464,33 @@ int solve_launch_count(const temf_ctx& c, int nrhs) {
   return (T.ntree ? 2 : 0) + (T.n_ftask ? 1 : 0) + (T.n_btask ? 1 : 0);
 }
 
-// Views of the sweeps through the ready queue: the single-column schedules
-// (q1) or the 64-row ones of the block sweeps (qm, backward accumulators in
-// place of the partial sums)
-static void queued_views(temf_ctx& c, bool block, double* const* Lbase, double* x, SweepView& vf, SweepView& vb) {
+// Views of the block sweeps (64-row schedules, backward accumulators in place
+// of the partial sums), with their ready queue.
+static void block_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& vf, SweepView& vb) {
   FactorPlan& F = c.fplan;
   SolvePlan& P = c.splan;
-  QueuePlan& Q = block ? P.qm : P.q1;
-  const int nf = block ? P.n_mftask : P.n_ftask, nb = block ? P.n_mbtask : P.n_btask;
+  QueuePlan& Q = P.qm;
+  const int nf = P.n_mftask, nb = P.n_mbtask;
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;  // fhead, bhead, ftail, btail
-  vf = SweepView{block ? P.mftask.p : P.ftask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x,
-                 block ? P.mftgt_ptr.p : P.ftgt_ptr.p, block ? P.mftgt.p : P.ftgt.p,
-                 block ? P.mfexpect.p : P.fexpect.p, nullptr, nullptr, nullptr, P.sync.p, P.nsn, nf,
+  vf = SweepView{P.mftask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.mftgt_ptr.p,
+                 P.mftgt.p, P.mfexpect.p, nullptr, nullptr, nullptr, P.sync.p, P.nsn, nf,
                  q, words + 0, words + 2, Q.fdiag.p, nullptr, nullptr, nullptr, nullptr, 0, Q.f_hi, 0,
                  c.spin_limit};
-  vb = SweepView{block ? P.mbtask.p : P.btask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x,
-                 block ? P.mbtgt_ptr.p : P.btgt_ptr.p, block ? P.mbtgt.p : P.btgt.p, nullptr,
-                 block ? P.mnchunk.p : P.nchunk.p, block ? P.macc_off.p : P.part_off.p, c.d_part.p, P.sync.p, P.nsn,
-                 nb, q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
+  vb = SweepView{P.mbtask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.mbtgt_ptr.p,
+                 P.mbtgt.p, nullptr, P.mnchunk.p, P.macc_off.p, c.d_part.p, P.sync.p, P.nsn, nb,
+                 q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
                  Q.b_lo, nb, 0, c.spin_limit};
-  vf.desc = block ? P.mfdesc.p : P.fdesc.p;
-  vb.desc = block ? P.mbdesc.p : P.bdesc.p;
+  vf.desc = P.mfdesc.p;
+  vb.desc = P.mbdesc.p;
   if (!uses_queue(Q, nb)) vf.queue = vb.queue = nullptr;
 }
 
 // clear the sweep words and seed both queues with their initially ready tasks
-static void reset_queues(temf_ctx& c, bool block, cudaStream_t st) {
+static void reset_block_queues(temf_ctx& c, cudaStream_t st) {
   SolvePlan& P = c.splan;
-  QueuePlan& Q = block ? P.qm : P.q1;
-  const int nf = block ? P.n_mftask : P.n_ftask, nb = block ? P.n_mbtask : P.n_btask;
+  QueuePlan& Q = P.qm;
+  const int nf = P.n_mftask, nb = P.n_mbtask;
   int* q = Q.qbuf.p;
   int* words = q + (size_t)nf + 2 * (size_t)nb;
   TEMF_CUDA(cudaMemsetAsync(P.sync.p, 0, P.sync_words() * sizeof(int), st));
@@ -2968,11 +2941,8 @@ int tune_solve(temf_ctx& c, int slot, int nrhs) {
   if (nrhs == 1) return tune_tree(c, slot);
   const Symbolic& S = c.sym;
   SolvePlan& P = c.splan;
-  const bool block = nrhs > 1;
-  QueuePlan& Q = block ? P.qm : P.q1;
+  QueuePlan& Q = P.qm;
   cudaStream_t st = c.stream;
-  Sched a;
-  if (!block) build_sched(S, kChunkRows, a);
   std::vector<int> cand = {0, level_below_width(S, 4096), level_below_width(S, 1024), level_below_width(S, 512),
                            level_below_width(S, 148), level_below_width(S, 32), S.nlevels};
   std::sort(cand.begin(), cand.end());
@@ -2994,8 +2964,7 @@ int tune_solve(temf_ctx& c, int slot, int nrhs) {
   int best = Q.split;
   double best_ms = 1e30;
   for (int sp : cand) {
-    if (block) upload_multi_plan(c, sp);
-    else upload_queue_plan(a, S, sp, Q, st);
+    upload_multi_plan(c, sp);
     double tot = 0.0;
     for (int rep = 0; rep < 4; ++rep) {
       TEMF_CUDA(cudaMemcpyAsync(x.p, ones.p, vec * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -3017,8 +2986,7 @@ int tune_solve(temf_ctx& c, int slot, int nrhs) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (block) upload_multi_plan(c, best);
-  else upload_queue_plan(a, S, best, Q, st);
+  upload_multi_plan(c, best);
   Q.tuned = true;
   return best;
 }
