@@ -152,7 +152,7 @@ struct BatchEngine {
       TEMF_CUDA(cudaMallocHost((void**)&R->err_h, 2 * sizeof(double)));
       for (int s = 0; s < 2; ++s)
         if (c.slots[s].L.n < (size_t)slot_len(c)) c.slots[s].L.alloc(slot_len(c));
-      ensure_update_buffer(c, 1);
+      ensure_chunk_sums(c);
       k_set_ptr_b<<<1, 1, 0, st>>>(R->lptr.p + 0, c.slots[0].L.p);
       k_set_ptr_b<<<1, 1, 0, st>>>(R->lptr.p + 1, c.slots[1].L.p);
       TEMF_CHECK_LAUNCH();

@@ -291,7 +291,7 @@ struct temf_ctx {
   temf::Source src;
   temf::Receivers rec;
   // scratch vectors
-  temf::DBuf<double> d_part;     // backward partial sums (part_len), or block accumulators (macc_len * 64)
+  temf::DBuf<double> d_part;     // backward chunk sums of a batch (part_len), or block accumulators (macc_len * 64)
   temf::AdjointRecord adj;
   temf::MeshFieldPlan mf;
   int u_nrhs = 0;

@@ -153,7 +153,7 @@ struct Engine {
     TEMF_CUDA(cudaMallocHost((void**)&err_h, 2 * nrhs * sizeof(double)));
     TEMF_CUDA(cudaEventCreate(&ev0));
     TEMF_CUDA(cudaEventCreate(&ev1));
-    ensure_update_buffer(c, nrhs);
+    if (nrhs > 1) ensure_block_sums(c);
     for (int s = 0; s < 2; ++s)
       if (c.slots[s].L.n < (size_t)slot_len(c)) c.slots[s].L.alloc(slot_len(c));
     k_set_ptr<<<1, 1, 0, st>>>(lptr.p + 0, c.slots[0].L.p);

@@ -2401,10 +2401,12 @@ void upload_multi_plan(temf_ctx& c, int split) {
   upload_queue_plan(b, S, split, P.qm, st);  // synchronises: the host vectors go out of scope
 }
 
-void ensure_update_buffer(temf_ctx& c, int nrhs) {
-  const SolvePlan& P = c.splan;
-  const size_t need = nrhs == 1 ? (size_t)std::max<int64_t>(P.part_len, 1)
-                                : (size_t)std::max<int64_t>(P.macc_len, 1) * kMultiCols;
+void ensure_block_sums(temf_ctx& c) {
+  const size_t need = (size_t)std::max<int64_t>(c.splan.macc_len, 1) * kMultiCols;
+  if (c.d_part.n < need) c.d_part.alloc(need);
+}
+void ensure_chunk_sums(temf_ctx& c) {
+  const size_t need = (size_t)std::max<int64_t>(c.splan.part_len, 1);
   if (c.d_part.n < need) c.d_part.alloc(need);
 }
 
@@ -2518,7 +2520,7 @@ static void tree_views(temf_ctx& c, double* const* Lbase, double* x, SweepView& 
                  q, words + 0, words + 2, Q.fdiag.p, nullptr, nullptr, nullptr, nullptr, 0, Q.f_hi, 0,
                  c.spin_limit};
   vb = SweepView{T.btask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, T.btgt_ptr.p,
-                 T.btgt.p, nullptr, P.nchunk.p, P.part_off.p, c.d_part.p, P.sync.p, P.nsn, nb,
+                 T.btgt.p, nullptr, P.nchunk.p, P.part_off.p, nullptr, P.sync.p, P.nsn, nb,
                  q + nf, words + 1, words + 3, Q.bdiag.p, Q.bdep_ptr.p, Q.bdep.p, Q.bneed.p, q + nf + nb,
                  Q.b_lo, nb, 0, c.spin_limit};
   vb.bacc = P.bacc();
@@ -2596,8 +2598,8 @@ void launch_residual(temf_ctx& c, const FactorSlot& fs, const double* x, const d
 
 void launch_solve(temf_ctx& c, double* const* Lbase, double* x, int nrhs, cudaStream_t st, const double* sgn) {
   SolvePlan& P = c.splan;
-  ensure_update_buffer(c, nrhs);
   if (nrhs > 1) {
+    ensure_block_sums(c);
     launch_solve_multi(c, Lbase, x, nrhs, st, sgn);
     return;
   }
@@ -2740,7 +2742,7 @@ SweepView bwd_view(temf_ctx& c, double* const* Lbase, double* x, int* sync, doub
   FactorPlan& F = c.fplan;
   SolvePlan& P = c.splan;
   if (!part) {
-    ensure_update_buffer(c, 1);
+    ensure_chunk_sums(c);
     part = c.d_part.p;
   }
   SweepView v{P.btask.p, F.sn_first.p, F.sn_rows_ptr.p, F.sn_rows.p, F.sn_Lptr.p, Lbase, x, P.btgt_ptr.p,

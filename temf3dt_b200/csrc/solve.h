@@ -49,7 +49,11 @@ void build_solve_plan(temf_ctx& c);
 // schedules replayed (both chunk heights; claim order and ready queue).
 // Empty string, or the violation.
 std::string check_schedules(const Symbolic& S);
-void ensure_update_buffer(temf_ctx& c, int nrhs);
+// The workspace of the backward sweeps that need one: the column sums of the
+// block sweeps, the chunk sums of the model batches (the single-column sweeps
+// sum into the plan's own words).
+void ensure_block_sums(temf_ctx& c);
+void ensure_chunk_sums(temf_ctx& c);
 
 // x (device, permuted order, row-major n x nrhs) is overwritten: b -> A^{-1} b.
 // `Lbase` points at a device word holding the panel base of the factor to use
