@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "dmma.cuh"
 #include "factor.h"
 
 namespace temf {
@@ -50,12 +51,6 @@ __global__ void k_load_A(int64_t n, const int* __restrict__ src, const int64_t* 
 // refinement of the solves recovers the accuracy.  The first non-positive
 // pivot is recorded in status[0] in both modes.
 constexpr double kPivotTol = 1e-13;
-
-__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 constexpr int kPotrfThreads = 256;  // warps 0-1: the panel's rows; the others: the columns after it, finished columns out
 constexpr int kPanel = 8;           // columns eliminated between two trailing updates

@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "factor.h"
+#include "dmma.cuh"
 #include "solve.h"
 
 namespace temf {
@@ -1238,12 +1239,6 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_bwd_models(int nstatic, co
 // ---------------------------------------------------------------------------
 constexpr int kLdm = 68;  // leading dimension of the 64-wide shared tiles: DMMA fragments without bank conflicts
 
-__device__ __forceinline__ void dmma8(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 
 struct alignas(16) MultiSmem {
   double D[kSnCols][kSnCols + 2];  // the diagonal block: forward transposed, [column][row]; backward [row][column]
@@ -1276,7 +1271,7 @@ __device__ __forceinline__ void mma_tile64(double (&acc)[2][NT][2], const double
 #pragma unroll
     for (int b = 0; b < NT; ++b)
 #pragma unroll
-      for (int a = 0; a < 2; ++a) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+      for (int a = 0; a < 2; ++a) dmma_8x8x4(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
   }
 }
 
@@ -1394,7 +1389,7 @@ __device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
 #pragma unroll
           for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 2; ++b) dmma8(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
+            for (int b = 0; b < 2; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
         }
 #pragma unroll
         for (int a = 0; a < 2; ++a)
