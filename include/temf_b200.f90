@@ -213,6 +213,10 @@ module temf_b200
       import; integer(c_int), value :: n; integer(c_long_long) :: xadj(*); integer(c_int) :: adj(*) 
       real(c_double) :: xyz(*); character(kind=c_char) :: msg(*); integer(c_int), value :: msg_len
     end function
+    integer(c_int) function temf_arith_check(ctx, which, n, a, b, out) bind(C, name="temf_arith_check")
+      import; type(c_ptr), value :: ctx; integer(c_int), value :: which; integer(c_int), value :: n 
+      real(c_double) :: a(*); real(c_double) :: b(*); real(c_double) :: out(*)
+    end function
     integer(c_int) function temf_pardiso_checker(symm, n, nnz, ia, ja, checker, msg, msg_len) &
         bind(C, name="temf_pardiso_checker")
       import; integer(c_int), value :: symm; integer(c_int), value :: n; integer(c_int), value :: nnz 

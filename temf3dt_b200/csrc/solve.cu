@@ -20,8 +20,8 @@
 //        tetrahedron (solution_output, src/FETD_FWD.f90:1532-1540).
 #include <algorithm>
 
-#include "factor.h"
 #include "dmma.cuh"
+#include "factor.h"
 #include "solve.h"
 
 namespace temf {
