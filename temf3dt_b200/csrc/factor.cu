@@ -865,6 +865,7 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   FactorPlan& F = c.fplan;
   FactorSlot& fs = c.slots[slot];
   cudaStream_t st = c.stream;
+  fs.valid = false;
   if (fs.L.n < (size_t)slot_len(c)) fs.L.alloc(slot_len(c));
   TEMF_CUDA(cudaMemsetAsync(fs.L.p, 0, S.stored * sizeof(double), st));
   int init[3] = {INT_MAX, 0, 0};
@@ -913,6 +914,15 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
   const cudaStream_t hi = W.chain;
   TEMF_CUDA(cudaEventRecord(W.chain_at, st));
   TEMF_CUDA(cudaStreamWaitEvent(hi, W.chain_at, 0));
+  // whatever ends the loop, the context's stream comes after what the chain runs
+  struct Join {
+    FactorStreams& W;
+    cudaStream_t st;
+    ~Join() {
+      cudaEventRecord(W.chain_at, W.chain);
+      cudaStreamWaitEvent(st, W.chain_at, 0);
+    }
+  } join{W, st};
   bool rest_pending = false;  // updates on st that the chain has not waited for
   for (int l = 0; l < S.nlevels; ++l) {
     const int cnt = S.level_ptr[l + 1] - S.level_ptr[l];
@@ -942,10 +952,7 @@ void launch_factor_values(temf_ctx& c, int slot, const double* X, double a, cons
       rest_pending = true;
     }
   }
-  TEMF_CUDA(cudaEventRecord(W.chain_at, hi));
-  TEMF_CUDA(cudaStreamWaitEvent(st, W.chain_at, 0));
   fs.dt = b * 0.5;
-  fs.valid = false;
 }
 
 }  // namespace temf
