@@ -21,8 +21,8 @@ struct Pattern {
   std::vector<int> contrib_idx;  // packed element entry: k * n_tets + t, k in [0,21)
 };
 
-// One entry of the factor update schedule: a 64x64 tile (rows i0.., cols j0..)
-// of the Schur update L21 * L21^T of supernode s (indices into its row list),
+// One entry of the factor update schedule: a tile (rows i0.., cols j0.., 64 or
+// 32 of each: the launch's shape) of the Schur update L21 * L21^T of supernode s (indices into its row list),
 // summed over the m = mj & 15 supernodes s-m+1 .. s (a run of column blocks
 // of one wider supernode), restricted to columns j < mj >> 4 when that is > 0.
 struct UpdTile {
@@ -47,7 +47,8 @@ struct FactorPlan {
   DBuf<int64_t> grp_relind;    // rel index of row 0 of the source (tables shared by the blocks of a run)
   DBuf<int> relind;
   DBuf<UpdTile> tiles;
-  // host, two parts per level: the tiles that the next level waits for, the others
+  // host, two parts per level: the tiles that the next level waits for, the
+  // others (on levels whose supernodes share no entry; else all in the first)
   struct UpdPart {
     int64_t first = 0, count = 0;
     int shape = 0;             // of the update kernel (factor.cu)
@@ -55,7 +56,7 @@ struct FactorPlan {
   std::vector<UpdPart> upd;
   DBuf<int2> trsm;             // (supernode, first row) chunks of the row solves
   std::vector<int64_t> trsm_level_ptr;
-  std::vector<int> level_width;  // host: widest supernode with rows below its block, per level
+  std::vector<int> level_width;  // host: widest supernode per level
   int64_t n_trsm = 0;
   int64_t n_relind = 0;
   int64_t n_tiles = 0;
@@ -77,14 +78,14 @@ struct SolveTask {
   int r1;
 };
 
-// What a single-column sweep task reads of the plan, in one 64-byte fetch (the
-// supernode's arrays are two dependent loads away from a SolveTask).
+// What a sweep task reads of the plan, in one 64-byte fetch (the supernode's
+// arrays are two dependent loads away from a SolveTask).
 struct alignas(16) TaskDesc {
   int s, kind, r0, r1;         // as SolveTask
   int f, c, ld, nchunk;        // first column, width, panel rows, row chunks of the supernode
   int tgt0, ntgt;              // forward: its targets in the target list; backward: the owner it waits for, 0 or 1
   int64_t panel;               // offset of row r0 of the rows below the block, from the panel base
-  int64_t diag;                // offset of the scaled copy of the block
+  int64_t diag;                // offset of the block as the sweep reads it: its scaled copy, or (block sweeps) the panel's
   int64_t rows;                // index of row r0 in the row lists
 };
 static_assert(sizeof(TaskDesc) == 64, "one task descriptor is four 16-byte loads");

@@ -11,14 +11,15 @@
 //   k_trsm       : the below-diagonal rows solved against it, 64 rows per
 //                  CTA, 16 columns at a time;
 //   k_update     : the Schur update L21 L21^T of every supernode of the level,
-//                  in 64x64 tiles on the FP64 tensor cores (DMMA
+//                  in tiles of 64x64 or 32x32 on the FP64 tensor cores (DMMA
 //                  mma.sync.m8n8k4.f64), scattered into the ancestor panels
-//                  through precomputed relative indices.  Several supernodes
-//                  of one level may update the same ancestor entry, so the
-//                  scatter of such levels uses FP64 atomics
-//                  (red.global.add.f64); a level holding a single supernode
-//                  (the dense top of the tree, where most flops are) writes
-//                  with plain read-modify-write.
+//                  through precomputed relative indices with FP64 atomics
+//                  (red.global.add.f64), on every level: launches overlap.
+// Supernodes of one level may update the same ancestor entry, in the order in
+// which their tiles finish: the last bit of such an entry differs from run to
+// run, and through the air's 1e-12 S/m so do the edge vectors, by 1e-9 to 1e-8
+// of their norm.  A level without such entries runs its updates in two launches
+// on two streams, behind the next level's blocks (launch_factor_values).
 // Pivot failures are reported through a status word (first failing column),
 // never by trapping.
 #include <algorithm>
@@ -254,7 +255,7 @@ constexpr unsigned kQuotientKey = ((1023u - 400u) << 20) - 1u;
 // start from the panel's entries (each entry gets its FMAs in ascending
 // column order, as in a row-by-row substitution), then one thread per row
 // substitutes inside the panel in registers.  A level of one 64-column block
-// takes 12.5 us where one row per thread and a division per column took 36.
+// takes 13 us where one row per thread and a division per column took 36.
 struct TrsmChunk {
   int s;
   int r0;
@@ -466,13 +467,13 @@ __device__ __forceinline__ void mbar_wait(uint64_t* b, unsigned parity, int* err
 //
 // Tile size and buffers go by the tiles launched together (update_shape).
 // More than one wave of 64 x 64 tiles with four buffers (three CTAs per SM):
-// two buffers and five CTAs per SM, bound by the FP64 tensor pipe (301k edges:
-// 18.3 ms a factorisation with the line at 3 tiles per SM, 18.8 at 8).  Up to
-// one wave is bound by the latency of a tile, and four buffers hide the
-// copies'.  Fewer tiles than SMs: 32 x 32 tiles, four times as many and a
-// quarter as long (a tile of 512 columns on its own: 83 us with two buffers
-// and a read-modify-write scatter, 49 as 32 x 32 tiles).  An entry's sum runs
-// over the same columns in the same order in every shape.
+// two buffers and five CTAs per SM, bound by the FP64 tensor pipe (27k edges
+// 1.58 ms a factorisation with the line at 3 tiles per SM, 1.62 at 8; 301k
+// 19.0 and 19.1).  Up to one wave is bound by the latency of a tile, and four
+// buffers hide the copies'.  Fewer tiles than SMs: 32 x 32 tiles, four times as
+// many and a quarter as long (a tile of 512 columns on its own: 83 us with two
+// buffers and a read-modify-write scatter, 49 as 32 x 32 tiles).  An entry's sum
+// runs over the same columns in the same order in every shape.
 constexpr int kUpdChunk = 16;
 
 template <int kT, int kStages>

@@ -854,8 +854,7 @@ __device__ __forceinline__ void sweep_tasks(const SweepView& V, ClaimSlots& S, i
 // With run leaders no task is claimed ahead: a leader waits for tasks claimed
 // after it, which must not be held back behind another.  The leader code needs
 // many more registers: without it both sweeps keep three CTAs per SM (168
-// registers; with two, without a spill, the backward sweep of the 1.48M-edge
-// mesh took 9.0 ms against 7.2 at three with spills), the backward sweep with
+// registers, no spills: the sweeps live off resident CTAs), the backward sweep with
 // leaders two.
 template <bool kLeaders, bool kForward>
 __device__ __forceinline__ void queued_sweep(const SweepView& V, int* err) {
@@ -1357,8 +1356,9 @@ __device__ __forceinline__ void store_rows(const double* Y, double* x, int64_t l
 // panel in registers.  Every entry gets its FMAs in the order of
 // column-by-column substitution (ascending going forward, descending going
 // backward: the fragments' four columns are taken in reverse there), so the
-// result does not depend on the panel width.  64 rows and columns: about 2 us;
-// column by column in shared memory it was 20, most of a level.
+// result does not depend on the panel width.  64 rows: 8 thousand
+// cycles (4 us) at 16 and at 64 columns; column by column in shared memory it was
+// 20 us, most of a level.
 template <bool kForward>
 __device__ __forceinline__ void diag_solve_block(MultiSmem& M, int c, int k) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -1615,8 +1615,10 @@ __global__ void __launch_bounds__(256) k_bdf_rhs(int n, const int* __restrict__ 
 
 // y = M x for one column in the caller's numbering (perm[row] = its index
 // there): the product with both permutations in one launch, eight lanes per
-// row (150k edges: 0.36 ms a host call against 0.39 with three launches, one thread
-// per row).
+// row, bound by the gathers.  Device time 3.4 us at 7k edges, 12.0 at 150k and 22
+// at 301k, against 10, 18.5 and 34 with two permutations around one thread per
+// row; a host call on pageable vectors 0.059, 0.37 and 0.63 ms against 0.066,
+// 0.384 and 0.68.
 __global__ void __launch_bounds__(256) k_spmv_user(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
                                                    const int* __restrict__ perm, const double* __restrict__ M,
                                                    const double* __restrict__ x, double* __restrict__ y) {

@@ -41,7 +41,7 @@ struct SweepView {
   // run leaders: offsets (from the panel base) of the factor's scaled copies
   // of the diagonal blocks (unit lower triangle, reciprocal diagonal)
   const int64_t* Dptr = nullptr;
-  const TaskDesc* desc = nullptr;  // single column: per task, all that it reads of the plan
+  const TaskDesc* desc = nullptr;  // per task, all that it reads of the plan
 };
 
 void build_solve_plan(temf_ctx& c);
